@@ -58,9 +58,10 @@ def reference_dir():
 
 def build_ref(ref_root: str | None = None) -> bool:
     """Compile the reference harness from the tree `ref_root` (default
-    $XDG_REFERENCE_DIR); False when no tree is given or it is absent."""
+    $XDG_REFERENCE_DIR); False when no tree is given or its sources are
+    absent."""
     ref_root = ref_root or reference_dir()
-    if not ref_root or not os.path.isdir(ref_root):
+    if not ref_root or not os.path.isfile(os.path.join(ref_root, "src", "geometry", "closest.cpp")):
         return False
     subprocess.run(["make", "-s", "-C", HERE, "ref", f"REF={ref_root}"], check=True)
     if not os.path.exists(REF_PATH):
