@@ -30,6 +30,7 @@
 #include "../../include/xdgcu.h"
 #include "bvh.h"
 #include "cbound.h"
+#include "imul64.cuh"
 #include "queries.h"
 #include "segments.h"
 #include "walk.h"
@@ -372,6 +373,7 @@ struct xdgcu_ctx {
   // edge table for the mixed walk's FP64 face tests (build_edge_table)
   DevMem<double> d_edge;
   DevMem<int32_t> d_tet_edge;
+  int32_t tet_int_ok = 0;  // every vertex coordinate is in_range() (imul64.cuh)
   int64_t n_edges = 0;
   DevMem<int32_t> d_elem_ids;
   int32_t face[12] = {0};
@@ -1253,6 +1255,7 @@ const char* walk_args_for(const xdgcu_ctx* c, WalkArgs* a, int* face_order, int*
   a->xyz32 = c->d_xyz32.p;
   a->edge = c->walk_edge_table ? c->d_edge.p : nullptr;
   a->tet_edge = c->d_tet_edge.p;
+  a->int_ok = c->tet_int_ok;
   a->conn = c->d_conn.p;
   a->adj = c->d_adj.p;
   a->elem_ids = c->d_elem_ids.p;
@@ -1451,6 +1454,9 @@ int xdgcu_set_tet_mesh(xdgcu_ctx* c, int64_t n_vertices, const double* xyz, int6
     if (adj[i] < -1 || adj[i] >= n_tets)
       return set_err(XDGCU_ERR_INVALID_ARG, "set_tet_mesh: adjacency out of range");
   }
+  c->tet_int_ok = 1;
+  for (int64_t i = 0; i < 3 * n_vertices; ++i)
+    if (!in_range(xyz[i])) c->tet_int_ok = 0;
   c->n_vert = n_vertices;
   c->n_tet = n_tets;
   API_CUDA(c->d_xyz.alloc(std::max<int64_t>(1, 3 * n_vertices)), "alloc vertices");
@@ -2185,6 +2191,7 @@ static int walk_query(xdgcu_ctx* c, bool walk, int64_t n, const int32_t* start, 
   a.xyz32 = c->d_xyz32.p;
   a.edge = c->walk_edge_table ? c->d_edge.p : nullptr;
   a.tet_edge = c->d_tet_edge.p;
+  a.int_ok = c->tet_int_ok;
   a.conn = c->d_conn.p;
   a.adj = c->d_adj.p;
   a.elem_ids = c->d_elem_ids.p;
@@ -2282,6 +2289,7 @@ int xdgcu_walk_elements_packed(xdgcu_ctx* c, int64_t n, const int32_t* start_ind
   a.xyz32 = c->d_xyz32.p;
   a.edge = c->walk_edge_table ? c->d_edge.p : nullptr;
   a.tet_edge = c->d_tet_edge.p;
+  a.int_ok = c->tet_int_ok;
   a.conn = c->d_conn.p;
   a.adj = c->d_adj.p;
   a.elem_ids = c->d_elem_ids.p;
@@ -2879,6 +2887,7 @@ int xdgcu_transport_elements(xdgcu_ctx* c, int64_t n, int32_t* elem_index, doubl
   a.xyz32 = c->d_xyz32.p;
   a.edge = c->walk_edge_table ? c->d_edge.p : nullptr;
   a.tet_edge = c->d_tet_edge.p;
+  a.int_ok = c->tet_int_ok;
   a.conn = c->d_conn.p;
   a.adj = c->d_adj.p;
   a.elem_ids = c->d_elem_ids.p;

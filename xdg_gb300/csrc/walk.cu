@@ -7,14 +7,20 @@
 // (element id, min(exit, remaining)) -- zero-length segments included -- and
 // moves r += len * u in FP64, exactly like :117-133.
 //
-// The FP64 variant evaluates all four faces with plucker64.  The mixed
+// The FP64 variant evaluates the tet's six edge coordinates in FP64 and takes
+// the distance to the faces their signs leave.  The mixed
 // variant first evaluates the six edge coordinates of the tet once in FP32
 // (each face uses three of them, with a sign flip when it runs an edge
 // backwards -- the exact coordinates of opposite directions are exact
 // negatives) and skips a face only when some coordinate is certainly
 // positive, which makes the FP64 test exit early (plucker.h:83-113).  The
-// remaining faces -- normally just the exit face -- are evaluated with
-// plucker64, so lengths and element sequences are bit-identical.
+// remaining faces -- normally just the exit face -- are evaluated in FP64
+// with the reference's operations, so lengths and element sequences are
+// bit-identical.
+//
+// What bounds it: the FP64 unit, 39 ns a warp instruction.  The exact test of
+// the exit face is some 75 FP64 operations a step; the products among them
+// run on the integer pipes instead (imul64.cuh), beside the sums.
 //
 // FP32 bound for a tet (u = 2^-24, D = |u|_inf, W = max |v_k - r|_inf,
 // Av = max |v_k|_inf, A = Av + |r|_inf; vertices and r rounded to FP32
@@ -29,6 +35,7 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
+#include "imul64.cuh"
 #include "internal.cuh"
 #include "sample.cuh"
 
@@ -58,7 +65,8 @@ __device__ __forceinline__ T sel4(const T* v, int k) {
   return k == 0 ? v[0] : (k == 1 ? v[1] : (k == 2 ? v[2] : v[3]));
 }
 
-__device__ __forceinline__ float sel6(const float* v, int k) {
+template <typename T>
+__device__ __forceinline__ T sel6(const T* v, int k) {
   return k == 0 ? v[0]
                 : (k == 1 ? v[1] : (k == 2 ? v[2] : (k == 3 ? v[3] : (k == 4 ? v[4] : v[5]))));
 }
@@ -82,6 +90,16 @@ struct StepCnt {
   unsigned long long steps, esc;
 };
 
+// The edge from local vertex la to lb of a tet (its six edge references at
+// te): the edge's index, bit 31 set when the test runs it against first()
+// order (the reference negates the coordinate then, plucker.h:48).
+__device__ __forceinline__ int32_t edge_ref(const int32_t* te, int la, int lb) {
+  const int32_t ref = __ldg(&te[pair_index(la, lb)]);
+  const bool second_is_lo = ref < 0;
+  const bool la_is_lo = second_is_lo == (la > lb);
+  return (ref & 0x7fffffff) | (la_is_lo ? 0 : (int32_t)0x80000000);
+}
+
 // plucker64 for the face (l0, l1, l2) of tet `tet` (vertex indices ci), its
 // three edge coordinates taken from the mesh's edge table: the same values
 // plucker_edge64 computes from the vertices, for a third of the FP64
@@ -91,12 +109,8 @@ __device__ __forceinline__ bool plucker64_face_pre(const WalkArgs& a, int32_t te
                                                    d3 r, d3 u, d3 rn, double* t) {
   const int32_t* te = a.tet_edge + 6 * (int64_t)tet;
   auto coord = [&](int la, int lb) {
-    const int32_t ref = __ldg(&te[pair_index(la, lb)]);
-    // the test runs la -> lb; the reference keeps the sign when la's vertex
-    // is the edge's lo (first(va, vb), plucker.h:48)
-    const bool second_is_lo = ref < 0;
-    const bool la_is_lo = second_is_lo == (la > lb);
-    return plucker_edge_pre(a.edge + 6 * (int64_t)(ref & 0x7fffffff), !la_is_lo, u, rn);
+    const int32_t ref = edge_ref(te, la, lb);
+    return plucker_edge_pre(a.edge + 6 * (int64_t)(ref & 0x7fffffff), ref < 0, u, rn);
   };
   const double c0 = coord(l0, l1), c1 = coord(l1, l2), c2 = coord(l2, l0);
   const int idx = plucker_axis(u);
@@ -107,37 +121,175 @@ __device__ __forceinline__ bool plucker64_face_pre(const WalkArgs& a, int32_t te
                           true, 1, t);
 }
 
+// ---------------------------------------------------------------------------
+// The step's exact arithmetic with its products on the integer pipes
+// (imul64.cuh).  A step takes this path when the mesh's coordinates
+// (WalkArgs::int_ok), the track's direction and its position are in range;
+// any other step takes the *_hw functions, whose products run on the FP64
+// unit.  Those are not inlined: a predicated-off FP64 instruction holds the
+// FP64 unit like one that runs, so the path not taken has to stay behind a
+// real branch.  Per step (lone operations a warp, FP64 unit): mixed 81 -> 40,
+// FP64 396 -> 54.
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ bool in_range3(d3 v) {
+  return in_range(v.x) && in_range(v.y) && in_range(v.z);
+}
+
+__device__ __forceinline__ double dot3_i(d3 a, d3 b) {
+  return mul_int(a.x, b.x) + mul_int(a.y, b.y) + mul_int(a.z, b.z);
+}
+
+__device__ __forceinline__ d3 cross3_i(d3 a, d3 b) {
+  return mk3(mul_int(a.y, b.z) - mul_int(a.z, b.y), mul_int(a.z, b.x) - mul_int(a.x, b.z),
+             mul_int(a.x, b.y) - mul_int(a.y, b.x));
+}
+
+// plucker_edge_pre for a reference of edge_ref()
+__device__ __forceinline__ double edge_coord_i(const double* edge, int32_t ref, d3 u, d3 rn) {
+  const double* E = edge + 6 * (int64_t)(ref & 0x7fffffff);
+  const double2 a = __ldg(reinterpret_cast<const double2*>(E));
+  const double2 b = __ldg(reinterpret_cast<const double2*>(E + 2));
+  const double2 c = __ldg(reinterpret_cast<const double2*>(E + 4));
+  double pip = dot3_i(u, mk3(b.y, c.x, c.y)) + dot3_i(rn, mk3(a.x, a.y, b.x));
+  pip = __longlong_as_double(__double_as_longlong(pip) ^ ((long long)(ref & 0x80000000) << 32));
+  if (absbits(pip) < absbits(ZERO_TOL)) pip = 0.0;
+  return pip;
+}
+
+__device__ __noinline__ bool sum_above_one(double a, double b) { return dlt(1.0, a + b); }
+
+// plucker64_coords for the walk's call (orientation +1, distances 0 ..
+// INFTY), for coordinates that are all <= 0 and not all 0: max(0, distance),
+// or INFTY for no hit.  The weights are >= 0, and their sum is tested only
+// where it can exceed 1: w1 >= 2^-48 keeps w0 + w2 below 1, since the
+// weights' sum is within 6 eps of 1.
+__device__ __forceinline__ double face_distance_i(double c0, double c1, double c2, double v0i,
+                                                  double v1i, double v2i, double oi, double di) {
+  const double inv = 1.0 / (c0 + c1 + c2);
+  const double w0 = mul_int(c0, inv), w1 = mul_int(c1, inv), w2 = mul_int(c2, inv);
+  const double hit = (mul_int(w0, v2i) + mul_int(w1, v0i)) + mul_int(w2, v1i);
+  double t = (hit - oi) / di;
+  if (absbits(w1) < 0x3cf0000000000000ull && sum_above_one(w2, w0)) t = -1.0;
+  if (lt0(t) || dlt(INFTY, t)) return INFTY;
+  return gt0(t) ? t : 0.0;
+}
+
+// The exit distance through one face, as face_distance_i, from the edge
+// table with the products on the FP64 unit: edge references e0..e2 of
+// edge_ref(), vertex indices i0..i2.
+__device__ __noinline__ double face_exit_hw(const double* edge, const double* xyz, int32_t e0,
+                                            int32_t e1, int32_t e2, int32_t i0, int32_t i1,
+                                            int32_t i2, d3 r, d3 u) {
+  const d3 rn = cross3(u, r);
+  const double c0 = plucker_edge_pre(edge + 6 * (int64_t)(e0 & 0x7fffffff), e0 < 0, u, rn);
+  const double c1 = plucker_edge_pre(edge + 6 * (int64_t)(e1 & 0x7fffffff), e1 < 0, u, rn);
+  const double c2 = plucker_edge_pre(edge + 6 * (int64_t)(e2 & 0x7fffffff), e2 < 0, u, rn);
+  const int idx = plucker_axis(u);
+  double t;
+  const bool hit =
+      plucker64_coords(c0, c1, c2, __ldg(&xyz[3 * (int64_t)i0 + idx]),
+                       __ldg(&xyz[3 * (int64_t)i1 + idx]), __ldg(&xyz[3 * (int64_t)i2 + idx]),
+                       comp3(r, idx), comp3(u, idx), INFTY, 0.0, true, 1, &t);
+  return hit ? (gt0(t) ? t : 0.0) : INFTY;
+}
+
+// the same from the vertices (a mesh without an edge table)
+__device__ __noinline__ double face_exit_xyz(const double* xyz, int32_t i0, int32_t i1, int32_t i2,
+                                             d3 r, d3 u) {
+  double t;
+  const bool hit = plucker64(load3(xyz, i0), load3(xyz, i1), load3(xyz, i2), r, u, cross3(u, r),
+                             INFTY, 0.0, true, 1, &t);
+  return hit ? (gt0(t) ? t : 0.0) : INFTY;
+}
+
+__device__ __noinline__ d3 move_hw(d3 r, double len, d3 u) { return add3(r, scl3(len, u)); }
+
+// r += len * u (mesh_manager_interface.cpp:133), safe as in next_face
+__device__ __forceinline__ d3 walk_move(d3 r, double len, d3 u, bool safe) {
+  // (a remaining distance can be any double: keep len * u normal)
+  const uint32_t h = words(len).hi;
+  if (safe && (h - (223u << 20) < (1200u << 20) || is0(len)))
+    return add3(r, mk3(mul_int(len, u.x), mul_int(len, u.y), mul_int(len, u.z)));
+  return move_hw(r, len, u);
+}
+
+// FP32 value nearest to x (to even), by integer operations: a conversion
+// instruction holds the FP64 unit for 33 ns a warp.  Magnitudes below FLT_MIN
+// give 0 (an error below 2^-126, far inside the filter's absolute term).
+__device__ __forceinline__ float f32_near(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const unsigned long long q = b + 0x0fffffffull + ((b >> 29) & 1ull);
+  const unsigned hi = (unsigned)(q >> 32);
+  const unsigned e = (hi >> 20) & 0x7ffu;
+  const unsigned sign = (unsigned)(b >> 32) & 0x80000000u;
+  if (e <= 896u) return __uint_as_float(sign);
+  if (e >= 1151u) return __uint_as_float(sign | 0x7f800000u);
+  return __uint_as_float(sign | ((unsigned)(q >> 29) - (896u << 23)) & 0x7fffffffu);
+}
+
+// What a step needs of the track's direction, set when it changes.
+struct StepDir {
+  float x, y, z;  // FP32, nearest
+  int axis;       // plucker_axis
+  bool safe;      // the mesh and the direction are in range (imul64.cuh)
+};
+
+__device__ __forceinline__ StepDir step_dir(const WalkArgs& a, d3 u) {
+  StepDir s;
+  s.x = f32_near(u.x);
+  s.y = f32_near(u.y);
+  s.z = f32_near(u.z);
+  s.axis = plucker_axis(u);
+  s.safe = a.edge && a.int_ok && in_range3(u);
+  return s;
+}
+
 // MeshManager::next_element for tet `elem` at r along u.  Returns the face
 // index (or -1) and writes the exit distance.
 template <int FO, bool MIXED>
 __device__ __forceinline__ int next_face(const WalkArgs& a, int32_t elem, d3 r, d3 u,
-                                         double* exit_dist, StepCnt& cnt) {
+                                         const StepDir& sd, bool safe, double* exit_dist,
+                                         StepCnt& cnt) {
   const int4 c = __ldg(&a.conn[elem]);
   const int32_t ci[4] = {c.x, c.y, c.z, c.w};
-  const d3 rn = cross3(u, r);  // plucker.h:75
-  double dists[4];
+  const int32_t* te = a.tet_edge + 6 * (int64_t)elem;
+  // the faces that may be the exit face: only these take the distance below
+  unsigned escm = 0u;
+  d3 rn = mk3(0.0, 0.0, 0.0);
+  double pe[6];  // FP64 path: the six coordinates, pair (i, j), i < j, run i -> j
+  if (safe) rn = cross3_i(u, r);  // plucker.h:75
   if (!MIXED) {
-    d3 V[4];
+    escm = 0xfu;
+    if (safe) {
+      escm = 0u;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) V[k] = load3(a.xyz, ci[k]);
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int f = 0; f < 4; ++f) {
-      const d3 f0 = sel4(V, face_local<FO>(a, f, 0));
-      const d3 f1 = sel4(V, face_local<FO>(a, f, 1));
-      const d3 f2 = sel4(V, face_local<FO>(a, f, 2));
-      double t;
-      const bool hit = plucker64(f0, f1, f2, r, u, rn, INFTY, 0.0, true, 1, &t);
-      dists[f] = hit ? (gt0(t) ? t : 0.0) : INFTY;  // std::max(0.0, t)
+        for (int j = i + 1; j < 4; ++j)
+          pe[pair_index(i, j)] = edge_coord_i(a.edge, edge_ref(te, i, j), u, rn);
+#pragma unroll
+      for (int f = 0; f < 4; ++f) {
+        const int l[3] = {face_local<FO>(a, f, 0), face_local<FO>(a, f, 1),
+                          face_local<FO>(a, f, 2)};
+        bool out = false, zero = true;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          const int la = l[q], lb = l[(q + 1) % 3];
+          const double p = sel6(pe, pair_index(la, lb));
+          out |= la < lb ? gt0(p) : lt0(p);  // a positive coordinate rejects (plucker.h:83-113)
+          zero &= is0(p);
+        }
+        if (!out && !zero) escm |= 1u << f;
+      }
     }
     cnt.esc += 4;
   } else {
     float4 P[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) P[k] = __ldg(&a.xyz32[ci[k]]);
-    const float rx = __double2float_rn(r.x), ry = __double2float_rn(r.y),
-                rz = __double2float_rn(r.z);
-    const float ux = __double2float_rn(u.x), uy = __double2float_rn(u.y),
-                uz = __double2float_rn(u.z);
+    const float rx = f32_near(r.x), ry = f32_near(r.y), rz = f32_near(r.z);
+    const float ux = sd.x, uy = sd.y, uz = sd.z;
     float wx[4], wy[4], wz[4];
     float W = 0.0f, Av = 0.0f;
 #pragma unroll
@@ -153,62 +305,68 @@ __device__ __forceinline__ int next_face(const WalkArgs& a, int32_t elem, d3 r, 
     const float thr =
         kU32 * 1.000001f * D * W * (97.0f * W + 13.0f * Av + 13.0f * A) * 1.0001f + 4.5e-15f;
     // pip(i -> j) = u . ((v_j - v_i) x (v_i - r)) for the six pairs i < j
-    float pe[6];
+    float pf[6];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = i + 1; j < 4; ++j)
-        pe[pair_index(i, j)] = triple32(ux, uy, uz, P[j].x - P[i].x, P[j].y - P[i].y,
+        pf[pair_index(i, j)] = triple32(ux, uy, uz, P[j].x - P[i].x, P[j].y - P[i].y,
                                         P[j].z - P[i].z, wx[i], wy[i], wz[i]);
     // faces whose FP32 coordinates do not certify an early exit
-    unsigned escm = 0u;
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
       const int l0 = face_local<FO>(a, f, 0), l1 = face_local<FO>(a, f, 1),
                 l2 = face_local<FO>(a, f, 2);
       const int e0 = pair_index(l0, l1), e1 = pair_index(l1, l2), e2 = pair_index(l2, l0);
-      const float p0 = l0 < l1 ? sel6(pe, e0) : -sel6(pe, e0);
-      const float p1 = l1 < l2 ? sel6(pe, e1) : -sel6(pe, e1);
-      const float p2 = l2 < l0 ? sel6(pe, e2) : -sel6(pe, e2);
+      const float p0 = l0 < l1 ? sel6(pf, e0) : -sel6(pf, e0);
+      const float p1 = l1 < l2 ? sel6(pf, e1) : -sel6(pf, e1);
+      const float p2 = l2 < l0 ? sel6(pf, e2) : -sel6(pf, e2);
       if (!(p0 > thr || p1 > thr || p2 > thr)) escm |= 1u << f;
     }
-    // FP64 for the remaining faces, in increasing face order (the strict-<
-    // argmin below is then the reference's, :191-196).  Every lane runs its
-    // first escalated face in the same iteration, so the FP64 work of a warp
-    // is issued once for all lanes.
-    int idx = -1;
-    double best = INFTY;
-    while (escm) {
-      const int f = __ffs(escm) - 1;
-      escm &= escm - 1u;
-      cnt.esc++;
-      const int l0 = face_local<FO>(a, f, 0), l1 = face_local<FO>(a, f, 1),
-                l2 = face_local<FO>(a, f, 2);
-      double t;
-      bool hit;
-      if (a.edge) {
-        hit = plucker64_face_pre(a, elem, ci, l0, l1, l2, r, u, rn, &t);
-      } else {
-        const d3 f0 = load3(a.xyz, sel4(ci, l0));
-        const d3 f1 = load3(a.xyz, sel4(ci, l1));
-        const d3 f2 = load3(a.xyz, sel4(ci, l2));
-        hit = plucker64(f0, f1, f2, r, u, rn, INFTY, 0.0, true, 1, &t);
-      }
-      const double df = hit ? (gt0(t) ? t : 0.0) : INFTY;  // std::max(0.0, t)
-      if (dlt(df, best)) {
-        best = df;
-        idx = f;
-      }
-    }
-    *exit_dist = best;
-    return idx;
   }
+  // The distance to the remaining faces, in increasing face order (the
+  // strict-< argmin is then the reference's, :191-196).  Every lane runs its
+  // first remaining face in the same iteration, so the FP64 work of a warp is
+  // issued once for all lanes.
   int idx = -1;
   double best = INFTY;
-#pragma unroll
-  for (int f = 0; f < 4; ++f) {
-    if (dlt(dists[f], best)) {
-      best = dists[f];
+  while (escm) {
+    const int f = __ffs(escm) - 1;
+    escm &= escm - 1u;
+    if (MIXED) cnt.esc++;
+    const int l0 = face_local<FO>(a, f, 0), l1 = face_local<FO>(a, f, 1),
+              l2 = face_local<FO>(a, f, 2);
+    const int32_t i0 = sel4(ci, l0), i1 = sel4(ci, l1), i2 = sel4(ci, l2);
+    double df = INFTY;
+    if (safe) {
+      double c0, c1, c2;
+      if (MIXED) {
+        c0 = edge_coord_i(a.edge, edge_ref(te, l0, l1), u, rn);
+        c1 = edge_coord_i(a.edge, edge_ref(te, l1, l2), u, rn);
+        c2 = edge_coord_i(a.edge, edge_ref(te, l2, l0), u, rn);
+      } else {
+        // (negated where the face runs the pair backwards; 0 stays +0)
+        auto coord = [&](int la, int lb) {
+          const double p = sel6(pe, pair_index(la, lb));
+          return la < lb || is0(p) ? p : -p;
+        };
+        c0 = coord(l0, l1);
+        c1 = coord(l1, l2);
+        c2 = coord(l2, l0);
+      }
+      if (!(gt0(c0) || gt0(c1) || gt0(c2)) && !(is0(c0) && is0(c1) && is0(c2)))
+        df = face_distance_i(c0, c1, c2, __ldg(&a.xyz[3 * (int64_t)i0 + sd.axis]),
+                             __ldg(&a.xyz[3 * (int64_t)i1 + sd.axis]),
+                             __ldg(&a.xyz[3 * (int64_t)i2 + sd.axis]), comp3(r, sd.axis),
+                             comp3(u, sd.axis));
+    } else if (a.edge) {
+      df = face_exit_hw(a.edge, a.xyz, edge_ref(te, l0, l1), edge_ref(te, l1, l2),
+                        edge_ref(te, l2, l0), i0, i1, i2, r, u);
+    } else {
+      df = face_exit_xyz(a.xyz, i0, i1, i2, r, u);
+    }
+    if (dlt(df, best)) {
+      best = df;
       idx = f;
     }
   }
@@ -248,8 +406,9 @@ __device__ __forceinline__ void walk_end_state(const WalkArgs& a, int64_t i, d3 
 // lanes stepping until its chunk is exhausted (track lengths are
 // exponentially distributed, so one-track-per-lane would leave most lanes
 // idle behind the longest track of the warp).
-template <int FO, bool MIXED>
-__global__ void __launch_bounds__(kBlock) k_walk(WalkArgs a, int64_t chunk) {
+// SUM: the running length sum is wanted (WalkArgs::sum_out).
+template <int FO, bool MIXED, bool SUM>
+__global__ void __launch_bounds__(kBlock, 4) k_walk(WalkArgs a, int64_t chunk) {
   const int lane = threadIdx.x & 31;
   const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   // the warp's tracks: positions first + k * stride, k < count (a contiguous
@@ -268,6 +427,7 @@ __global__ void __launch_bounds__(kBlock) k_walk(WalkArgs a, int64_t chunk) {
   d3 r = mk3(0, 0, 0), u = mk3(0, 0, 0);
   double dist = 0.0, sum = 0.0;
   int32_t elem = -1, k = 0, st = RAY_OK;
+  StepDir sd = {};
   int32_t* oe = nullptr;
   double* ol = nullptr;
   while (true) {
@@ -284,8 +444,9 @@ __global__ void __launch_bounds__(kBlock) k_walk(WalkArgs a, int64_t chunk) {
           has = true;
           r = load3(a.org, i);
           u = load3(a.dir, i);
+          sd = step_dir(a, u);
           dist = a.dist[i];
-          sum = a.sum_in ? a.sum_in[i] : 0.0;
+          sum = SUM && a.sum_in ? a.sum_in[i] : 0.0;
           elem = a.start[i];
           k = 0;
           st = RAY_OK;
@@ -324,7 +485,8 @@ __global__ void __launch_bounds__(kBlock) k_walk(WalkArgs a, int64_t chunk) {
       if (!done) {
         cnt.steps++;
         double ex;
-        const int f = next_face<FO, MIXED>(a, elem, r, u, &ex, cnt);
+        const bool safe = sd.safe && in_range3(r);
+        const int f = next_face<FO, MIXED>(a, elem, r, u, sd, safe, &ex, cnt);
         int32_t nxt = -1;
         if (f < 0) {
           st = RAY_NO_EXIT_FACE;  // the reference would index adjacency with -1
@@ -334,13 +496,13 @@ __global__ void __launch_bounds__(kBlock) k_walk(WalkArgs a, int64_t chunk) {
         }
         ex = dlt(dist, ex) ? dist : ex;  // std::min(exit, distance)
         dist -= ex;
-        if (a.sum_out) sum = sum + ex;
+        if (SUM) sum = sum + ex;
         if (oe) {
           oe[k] = __ldg(&a.elem_ids[elem]);
           ol[k] = ex;
         }
         ++k;
-        r = add3(r, scl3(ex, u));  // r += exit.second * u
+        r = walk_move(r, ex, u, safe);  // r += exit.second * u
         if (nxt < -1 || nxt >= a.n_tets) {
           st = RAY_INVALID;  // corrupt adjacency: stop instead of reading out of range
           done = true;
@@ -381,7 +543,8 @@ __global__ void __launch_bounds__(kBlock) k_next(WalkArgs a) {
       st = RAY_INVALID;
     } else {
       cnt.steps++;
-      const int f = next_face<FO, MIXED>(a, elem, r, u, &ex, cnt);
+      const StepDir sd = step_dir(a, u);
+      const int f = next_face<FO, MIXED>(a, elem, r, u, sd, sd.safe && in_range3(r), &ex, cnt);
       if (f < 0) {
         st = RAY_NO_EXIT_FACE;
       } else {
@@ -816,10 +979,10 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_apply(int64_t* __restrict__
   if (blockIdx.x == 0 && threadIdx.x == 0) v[n] = sums[nb];
 }
 
-template <int FO, bool MIXED, bool QUEUE>
-cudaError_t launch_walk_t(const WalkArgs& a, cudaStream_t st) {
+template <int FO, bool MIXED, bool QUEUE, bool SUM>
+cudaError_t launch_walk_s(const WalkArgs& a, cudaStream_t st) {
   static std::atomic<int> cached[kMaxDevices];  // resident blocks per SM, per device
-  auto kern = QUEUE ? k_walk_q<FO> : k_walk<FO, MIXED>;
+  auto kern = QUEUE ? k_walk_q<FO> : k_walk<FO, MIXED, SUM>;
   int per_sm = 0;
   const cudaError_t e = occupancy_cached(cached, kern, kBlock, 0, per_sm);
   if (e != cudaSuccess) return e;
@@ -831,6 +994,12 @@ cudaError_t launch_walk_t(const WalkArgs& a, cudaStream_t st) {
   const int64_t chunk = (a.n + warps - 1) / warps;
   kern<<<(unsigned)blocks, kBlock, 0, st>>>(a, chunk);
   return cudaGetLastError();
+}
+
+template <int FO, bool MIXED, bool QUEUE>
+cudaError_t launch_walk_t(const WalkArgs& a, cudaStream_t st) {
+  return a.sum_out ? launch_walk_s<FO, MIXED, QUEUE, true>(a, st)
+                   : launch_walk_s<FO, MIXED, QUEUE, false>(a, st);
 }
 
 }  // namespace
@@ -869,7 +1038,7 @@ namespace {
 // ---------------------------------------------------------------------------
 
 template <int FO, bool MIXED>
-__global__ void __launch_bounds__(kBlock) k_transport(TransportArgs t, int64_t chunk) {
+__global__ void __launch_bounds__(kBlock, 4) k_transport(TransportArgs t, int64_t chunk) {
   const WalkArgs& a = t.mesh;
   const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   int64_t cursor = gwarp * chunk;
@@ -885,8 +1054,10 @@ __global__ void __launch_bounds__(kBlock) k_transport(TransportArgs t, int64_t c
   // an event whose FP64 part waits for the warp's batch: its uniform draw,
   // exit distance and exit face
   bool pend = false;
-  double pu = 0.0, pex = 0.0;
+  unsigned long long pu = 0ull;
+  double pex = 0.0;
   int pf = -1;
+  StepDir sd = {};
   const float mfp32 = (float)t.mfp;
   const bool quick = t.mfp < 1e30;
 
@@ -899,7 +1070,7 @@ __global__ void __launch_bounds__(kBlock) k_transport(TransportArgs t, int64_t c
     }
     const int4 ad = __ldg(&a.adj[elem]);
     const int32_t nxt = f == 0 ? ad.x : (f == 1 ? ad.y : (f == 2 ? ad.z : ad.w));
-    r = add3(r, scl3(ex, u));
+    r = walk_move(r, ex, u, sd.safe && in_range3(r));
     dist += ex;
     if (t.tally) atomicAdd(&t.tally[elem], ex);
     if (nxt < -1 || nxt >= a.n_tets) {
@@ -925,6 +1096,7 @@ __global__ void __launch_bounds__(kBlock) k_transport(TransportArgs t, int64_t c
           elem = t.elem[i];
           r = load3(t.pos, i);
           u = load3(t.dir, i);
+          sd = step_dir(a, u);
           rs = t.rng[i];
           dist = t.distance[i];
           ev = t.events[i];
@@ -945,15 +1117,16 @@ __global__ void __launch_bounds__(kBlock) k_transport(TransportArgs t, int64_t c
       if (!done) {
         cnt.steps++;
         double ex;
-        const int f = next_face<FO, MIXED>(a, elem, r, u, &ex, cnt);
-        const double U = uniform53(rs);
+        const int f = next_face<FO, MIXED>(a, elem, r, u, sd, sd.safe && in_range3(r), &ex, cnt);
+        // 1 - U of uniform53's U = k 2^-53 is (2^53 - k) 2^-53, exactly
+        const unsigned long long U = (1ull << 53) - (splitmix_next(rs) >> 11);
         // Most events leave the tet: an FP32 logarithm with a certified
         // margin decides c >= exit without the FP64 series.  |c32 - c| <=
         // 6.1e-8 mfp + 3.7e-7 c (rounding 1 - U to FP32, logf within 2 ulp,
         // two FP32 products); the margin below is 1.1e-6 (c32 + mfp).
         bool leaves = false;
         if (quick) {
-          const float c32 = -logf(__double2float_rn(1.0 - U)) * mfp32;
+          const float c32 = -logf(__ull2float_rn(U) * 1.1102230246251565e-16f) * mfp32;
           const float lo = c32 - 1.1e-6f * (c32 + mfp32);
           leaves = dlt(ex, (double)lo);  // c >= lo > exit
         }
@@ -976,13 +1149,15 @@ __global__ void __launch_bounds__(kBlock) k_transport(TransportArgs t, int64_t c
       if (__popc(pm) >= t.event_wait || run == 0u) {
         if (has && pend) {
           pend = false;
-          const double c = -series_log(1.0 - pu) * t.mfp;  // sample_collision's value
+          // sample_collision's value
+          const double c = -series_log((double)pu * 1.1102230246251565e-16) * t.mfp;
           if (dlt(c, pex)) {
             // collision inside the tet (:81-85)
-            r = add3(r, scl3(c, u));
+            r = walk_move(r, c, u, sd.safe && in_range3(r));
             dist += c;
             if (t.tally) atomicAdd(&t.tally[elem], c);
             u = sample_direction(rs);
+            sd = step_dir(a, u);
             ++ev;
           } else {
             done = exit_step(pex, pf);

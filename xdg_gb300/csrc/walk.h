@@ -19,6 +19,7 @@ struct WalkArgs {
   // bit 31 set when the pair's second vertex is the edge's lo
   const double* edge;
   const int32_t* tet_edge;
+  int32_t int_ok;        // every vertex coordinate is in_range() (imul64.cuh)
   int32_t n_tets;
   int32_t face[12];      // local face table
   int64_t n;
