@@ -369,10 +369,10 @@ struct xdgcu_ctx {
   int64_t n_vert = 0, n_tet = 0;
   DevMem<double> d_xyz;
   DevMem<float4> d_xyz32;
-  DevMem<int4> d_conn, d_adj;
+  DevMem<int4> d_conn;
+  DevMem<int4> d_rec;  // the walk's records (WalkArgs::rec)
   // edge table for the mixed walk's FP64 face tests (build_edge_table)
   DevMem<double> d_edge;
-  DevMem<int32_t> d_tet_edge;
   int32_t tet_int_ok = 0;  // every vertex coordinate is in_range() (imul64.cuh)
   int64_t n_edges = 0;
   DevMem<int32_t> d_elem_ids;
@@ -950,15 +950,18 @@ int with_length_order(xdgcu_ctx* c, WalkArgs& a, cudaStream_t s, Body body) {
   const size_t ord_bytes = ((sizeof(int32_t) * (size_t)a.n + 255) & ~(size_t)255);
   const size_t scr = walk_order_scratch_bytes(a.n);
   char* buf = nullptr;
-  API_CUDA(scratch_alloc(c, (void**)&buf, ord_bytes + scr, s), "walk order scratch");
-  cudaError_t e = walk_order(a.dist, a.n, (int32_t*)buf, buf + ord_bytes, scr, s);
+  API_CUDA(scratch_alloc(c, (void**)&buf, 256 + ord_bytes + scr, s), "walk order scratch");
+  int32_t* const order = (int32_t*)(buf + 256);
+  cudaError_t e = walk_order(a.dist, a.n, order, buf + 256 + ord_bytes, scr, s);
   if (e != cudaSuccess) {
     cudaFreeAsync(buf, s);
     return cuda_err(e, "walk order");
   }
-  a.order = (const int32_t*)buf;
+  a.order = order;
+  a.work = (unsigned long long*)buf;
   const int rc = body();
   a.order = nullptr;
+  a.work = nullptr;
   cudaFreeAsync(buf, s);
   return rc;
 }
@@ -1068,8 +1071,9 @@ int seg_walk_round(xdgcu_ctx* c, bool mixed, const SegState& ss, const WalkArgs&
   w.status = B.wst;
   w.seg_count = B.wcnt;
   w.stop_elem = B.wstop;
-  w.sum_in = B.wsum_in;
-  w.sum_out = B.wsum_out;
+  // (the packed walk has no use for the running sums)
+  w.sum_in = walk_only ? nullptr : B.wsum_in;
+  w.sum_out = walk_only ? nullptr : B.wsum_out;
   w.end_r = B.wend_r;
   w.end_dist = B.wend_d;
   w.seg_elem = B.sk_elem;
@@ -1093,7 +1097,7 @@ int seg_walk_round(xdgcu_ctx* c, bool mixed, const SegState& ss, const WalkArgs&
     return set_err(XDGCU_ERR_CUDA, "walk rounds: temporary memory");
   API_CUDA(seg_pack(m, K, B.sk_elem, B.sk_len, R->off, R->seg_elem, R->seg_len, st), "walk pack");
   API_CUDA(seg_advance(ss, R->walk_t, m, K, B.sk_elem, B.wcnt, B.wst, B.wstop, B.wend_r, B.wend_d,
-                       B.wsum_out, max_segs, R->off, R->dst_rel, act_next, n_act, st, walk_only),
+                       w.sum_out, max_segs, R->off, R->dst_rel, act_next, n_act, st, walk_only),
            "walk advance");
   return XDGCU_OK;
 }
@@ -1254,11 +1258,8 @@ const char* walk_args_for(const xdgcu_ctx* c, WalkArgs* a, int* face_order, int*
   a->xyz = c->d_xyz.p;
   a->xyz32 = c->d_xyz32.p;
   a->edge = c->walk_edge_table ? c->d_edge.p : nullptr;
-  a->tet_edge = c->d_tet_edge.p;
   a->int_ok = c->tet_int_ok;
-  a->conn = c->d_conn.p;
-  a->adj = c->d_adj.p;
-  a->elem_ids = c->d_elem_ids.p;
+  a->rec = c->d_rec.p;
   a->n_tets = (int32_t)c->n_tet;
   std::memcpy(a->face, c->face, sizeof(a->face));
   a->walk_queue = c->walk_queue;
@@ -1462,7 +1463,10 @@ int xdgcu_set_tet_mesh(xdgcu_ctx* c, int64_t n_vertices, const double* xyz, int6
   API_CUDA(c->d_xyz.alloc(std::max<int64_t>(1, 3 * n_vertices)), "alloc vertices");
   API_CUDA(c->d_xyz32.alloc(std::max<int64_t>(1, n_vertices)), "alloc vertices");
   API_CUDA(c->d_conn.alloc(std::max<int64_t>(1, n_tets)), "alloc tets");
-  API_CUDA(c->d_adj.alloc(std::max<int64_t>(1, n_tets)), "alloc tets");
+  API_CUDA(c->d_rec.alloc(std::max<int64_t>(1, 4 * n_tets)), "alloc tets");
+  DevMem<int4> adj_dev;
+  DevMem<int32_t> tet_edge_dev;
+  API_CUDA(adj_dev.alloc(std::max<int64_t>(1, n_tets)), "alloc tets");
   API_CUDA(c->d_elem_ids.alloc(std::max<int64_t>(1, n_tets)), "alloc tets");
   if (n_vertices) {
     API_CUDA(cudaMemcpy(c->d_xyz.p, xyz, sizeof(double) * 3 * n_vertices, cudaMemcpyHostToDevice),
@@ -1474,7 +1478,7 @@ int xdgcu_set_tet_mesh(xdgcu_ctx* c, int64_t n_vertices, const double* xyz, int6
   if (n_tets) {
     API_CUDA(cudaMemcpy(c->d_conn.p, conn, sizeof(int32_t) * 4 * n_tets, cudaMemcpyHostToDevice),
              "upload tets");
-    API_CUDA(cudaMemcpy(c->d_adj.p, adj, sizeof(int32_t) * 4 * n_tets, cudaMemcpyHostToDevice),
+    API_CUDA(cudaMemcpy(adj_dev.p, adj, sizeof(int32_t) * 4 * n_tets, cudaMemcpyHostToDevice),
              "upload tets");
     API_CUDA(cudaMemcpy(c->d_elem_ids.p, elem_ids, sizeof(int32_t) * n_tets, cudaMemcpyHostToDevice),
              "upload tets");
@@ -1489,10 +1493,13 @@ int xdgcu_set_tet_mesh(xdgcu_ctx* c, int64_t n_vertices, const double* xyz, int6
         cudaGetLastError();
       c->d_edge.p = edge;
       c->d_edge.n = 6 * ne;
-      c->d_tet_edge.p = tet_edge;
-      c->d_tet_edge.n = 6 * n_tets;
+      tet_edge_dev.p = tet_edge;
+      tet_edge_dev.n = 6 * n_tets;
       c->n_edges = ne;
     }
+    API_CUDA(build_tet_records(c->d_conn.p, adj_dev.p, tet_edge_dev.p, c->d_elem_ids.p, n_tets,
+                               c->d_rec.p, c->build_stream), "tet records");
+    API_CUDA(cudaStreamSynchronize(c->build_stream), "tet records");
   }
   std::memcpy(c->face, face_table, sizeof(c->face));
   c->face_order = std::memcmp(face_table, kMoabFaces, sizeof(kMoabFaces)) == 0 ? 0 : 1;
@@ -2190,11 +2197,8 @@ static int walk_query(xdgcu_ctx* c, bool walk, int64_t n, const int32_t* start, 
   a.xyz = c->d_xyz.p;
   a.xyz32 = c->d_xyz32.p;
   a.edge = c->walk_edge_table ? c->d_edge.p : nullptr;
-  a.tet_edge = c->d_tet_edge.p;
   a.int_ok = c->tet_int_ok;
-  a.conn = c->d_conn.p;
-  a.adj = c->d_adj.p;
-  a.elem_ids = c->d_elem_ids.p;
+  a.rec = c->d_rec.p;
   a.n_tets = (int32_t)c->n_tet;
   std::memcpy(a.face, c->face, sizeof(a.face));
   a.walk_queue = c->walk_queue;
@@ -2288,11 +2292,8 @@ int xdgcu_walk_elements_packed(xdgcu_ctx* c, int64_t n, const int32_t* start_ind
   a.xyz = c->d_xyz.p;
   a.xyz32 = c->d_xyz32.p;
   a.edge = c->walk_edge_table ? c->d_edge.p : nullptr;
-  a.tet_edge = c->d_tet_edge.p;
   a.int_ok = c->tet_int_ok;
-  a.conn = c->d_conn.p;
-  a.adj = c->d_adj.p;
-  a.elem_ids = c->d_elem_ids.p;
+  a.rec = c->d_rec.p;
   a.n_tets = (int32_t)c->n_tet;
   std::memcpy(a.face, c->face, sizeof(a.face));
   a.walk_queue = c->walk_queue;
@@ -2886,11 +2887,8 @@ int xdgcu_transport_elements(xdgcu_ctx* c, int64_t n, int32_t* elem_index, doubl
   a.xyz = c->d_xyz.p;
   a.xyz32 = c->d_xyz32.p;
   a.edge = c->walk_edge_table ? c->d_edge.p : nullptr;
-  a.tet_edge = c->d_tet_edge.p;
   a.int_ok = c->tet_int_ok;
-  a.conn = c->d_conn.p;
-  a.adj = c->d_adj.p;
-  a.elem_ids = c->d_elem_ids.p;
+  a.rec = c->d_rec.p;
   a.n_tets = (int32_t)c->n_tet;
   std::memcpy(a.face, c->face, sizeof(a.face));
   t.n = n;

@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kSegBlock) k_seg_advance(
   const int64_t kept = off[k + 1] - off[k];
   // std::accumulate(vol_segments, 0.0, ...) continued across pauses: the walk
   // kernel added this round's lengths, in order, to the sum it was given
-  const double sum = wsum[k];
+  const double sum = wsum ? wsum[k] : 0.0;
   dst_rel[k] = s.written[t];
   s.written[t] += kept;
   if (kept > 0) s.last[t] = seg_elem[k * (int64_t)K + kept - 1];

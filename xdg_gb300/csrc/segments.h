@@ -113,7 +113,7 @@ cudaError_t seg_pack(int64_t m, int32_t K, const int32_t* seg_elem, const double
 
 // After the round's walk (K-strided segments seg_elem, counts cnt, statuses
 // wst, and per walk entry where it stopped: element wstop, position wend_r,
-// distance left wend_d, running length sum wsum) and the scan of the kept
+// distance left wend_d, running length sum wsum, null with walk_only) and the scan of the kept
 // counts into off[0..m]: the walk state advanced, dst_rel[k] = the track's
 // segments written before this round; a walk that ends applies segment_sum
 // to r and distance; the tracks still active (paused or with distance left)

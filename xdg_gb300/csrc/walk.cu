@@ -86,15 +86,29 @@ __device__ __forceinline__ int pair_index(int i, int j) {
   return a == 0 ? b - 1 : (a == 1 ? b + 1 : 5);
 }
 
+// (32-bit: a thread's share of one launch stays far below 2^32)
 struct StepCnt {
-  unsigned long long steps, esc;
+  uint32_t steps, esc;
 };
+
+// A tet's record (WalkArgs::rec): its vertices, neighbours, edge references and
+// mesh id, 64 bytes in one line, so that a step fetches all it needs of the
+// tet at once instead of from four arrays.
+struct TetRec {
+  int32_t v[4], adj[4], edge[6], id;
+};
+
+__device__ __forceinline__ TetRec load_rec(const WalkArgs& a, int32_t elem) {
+  const int4* p = a.rec + 4 * (int64_t)elem;
+  const int4 v = __ldg(p), n = __ldg(p + 1), e = __ldg(p + 2), f = __ldg(p + 3);
+  return {{v.x, v.y, v.z, v.w}, {n.x, n.y, n.z, n.w}, {e.x, e.y, e.z, e.w, f.x, f.y}, f.z};
+}
 
 // The edge from local vertex la to lb of a tet (its six edge references at
 // te): the edge's index, bit 31 set when the test runs it against first()
 // order (the reference negates the coordinate then, plucker.h:48).
-__device__ __forceinline__ int32_t edge_ref(const int32_t* te, int la, int lb) {
-  const int32_t ref = __ldg(&te[pair_index(la, lb)]);
+__device__ __forceinline__ int32_t edge_ref(const int32_t te[6], int la, int lb) {
+  const int32_t ref = sel6(te, pair_index(la, lb));
   const bool second_is_lo = ref < 0;
   const bool la_is_lo = second_is_lo == (la > lb);
   return (ref & 0x7fffffff) | (la_is_lo ? 0 : (int32_t)0x80000000);
@@ -107,7 +121,8 @@ __device__ __forceinline__ int32_t edge_ref(const int32_t* te, int la, int lb) {
 __device__ __forceinline__ bool plucker64_face_pre(const WalkArgs& a, int32_t tet,
                                                    const int32_t ci[4], int l0, int l1, int l2,
                                                    d3 r, d3 u, d3 rn, double* t) {
-  const int32_t* te = a.tet_edge + 6 * (int64_t)tet;
+  const TetRec T = load_rec(a, tet);
+  const int32_t* te = T.edge;
   auto coord = [&](int la, int lb) {
     const int32_t ref = edge_ref(te, la, lb);
     return plucker_edge_pre(a.edge + 6 * (int64_t)(ref & 0x7fffffff), ref < 0, u, rn);
@@ -128,8 +143,8 @@ __device__ __forceinline__ bool plucker64_face_pre(const WalkArgs& a, int32_t te
 // any other step takes the *_hw functions, whose products run on the FP64
 // unit.  Those are not inlined: a predicated-off FP64 instruction holds the
 // FP64 unit like one that runs, so the path not taken has to stay behind a
-// real branch.  Per step (lone operations a warp, FP64 unit): mixed 81 -> 40,
-// FP64 396 -> 54.
+// real branch.  FP64 unit instructions a step: mixed 81 -> 43, FP64 396 -> 57
+// (r += len * u stays there: its three products made no difference).
 // ---------------------------------------------------------------------------
 
 __device__ __forceinline__ bool in_range3(d3 v) {
@@ -203,17 +218,6 @@ __device__ __noinline__ double face_exit_xyz(const double* xyz, int32_t i0, int3
   return hit ? (gt0(t) ? t : 0.0) : INFTY;
 }
 
-__device__ __noinline__ d3 move_hw(d3 r, double len, d3 u) { return add3(r, scl3(len, u)); }
-
-// r += len * u (mesh_manager_interface.cpp:133), safe as in next_face
-__device__ __forceinline__ d3 walk_move(d3 r, double len, d3 u, bool safe) {
-  // (a remaining distance can be any double: keep len * u normal)
-  const uint32_t h = words(len).hi;
-  if (safe && (h - (223u << 20) < (1200u << 20) || is0(len)))
-    return add3(r, mk3(mul_int(len, u.x), mul_int(len, u.y), mul_int(len, u.z)));
-  return move_hw(r, len, u);
-}
-
 // FP32 value nearest to x (to even), by integer operations: a conversion
 // instruction holds the FP64 unit for 33 ns a warp.  Magnitudes below FLT_MIN
 // give 0 (an error below 2^-126, far inside the filter's absolute term).
@@ -245,15 +249,14 @@ __device__ __forceinline__ StepDir step_dir(const WalkArgs& a, d3 u) {
   return s;
 }
 
-// MeshManager::next_element for tet `elem` at r along u.  Returns the face
+// MeshManager::next_element for the tet of record T at r along u.  Returns the face
 // index (or -1) and writes the exit distance.
 template <int FO, bool MIXED>
-__device__ __forceinline__ int next_face(const WalkArgs& a, int32_t elem, d3 r, d3 u,
+__device__ __forceinline__ int next_face(const WalkArgs& a, const TetRec& T, d3 r, d3 u,
                                          const StepDir& sd, bool safe, double* exit_dist,
                                          StepCnt& cnt) {
-  const int4 c = __ldg(&a.conn[elem]);
-  const int32_t ci[4] = {c.x, c.y, c.z, c.w};
-  const int32_t* te = a.tet_edge + 6 * (int64_t)elem;
+  const int32_t* ci = T.v;
+  const int32_t* te = T.edge;
   // the faces that may be the exit face: only these take the distance below
   unsigned escm = 0u;
   d3 rn = mk3(0.0, 0.0, 0.0);
@@ -323,6 +326,13 @@ __device__ __forceinline__ int next_face(const WalkArgs& a, int32_t elem, d3 r, 
       const float p2 = l2 < l0 ? sel6(pf, e2) : -sel6(pf, e2);
       if (!(p0 > thr || p1 > thr || p2 > thr)) escm |= 1u << f;
     }
+  }
+  // the neighbour behind the (normally only) remaining face is the next step's
+  // tet: its record comes in while this step's arithmetic runs
+  if (escm) {
+    const int32_t nx = sel4(T.adj, __ffs(escm) - 1);
+    if (nx >= 0 && nx < a.n_tets)
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(a.rec + 4 * (int64_t)nx));
   }
   // The distance to the remaining faces, in increasing face order (the
   // strict-< argmin is then the reference's, :191-196).  Every lane runs its
@@ -401,25 +411,55 @@ __device__ __forceinline__ void walk_end_state(const WalkArgs& a, int64_t i, d3 
   if (a.end_dist) a.end_dist[i] = dist;
 }
 
-// Persistent walk: each warp owns a contiguous chunk of tracks; a lane whose
-// track has ended takes the next track of the chunk, so a warp keeps all 32
-// lanes stepping until its chunk is exhausted (track lengths are
-// exponentially distributed, so one-track-per-lane would leave most lanes
-// idle behind the longest track of the warp).
+// Where a warp's tracks come from: positions cursor .. end - 1 of the batch,
+// or of the length order.  Without an order, one contiguous chunk.  With one,
+// the warp takes 32 consecutive positions at a time, longest first, from the
+// launch's work counter.  The lanes of a warp then hold tracks of about the
+// same length and end together, so the FP64 unit, which takes as long for one
+// lane as for 32, sees full warps (dealt one by one, every warp held one of
+// the longest tracks and stepped on for it alone), and the warps end together
+// too (dealt in fixed shares, the SMs were idle a fifth of the launch on
+// 3e5 tracks).
+struct WarpTracks {
+  int64_t cursor, end;
+  __device__ __forceinline__ WarpTracks(const WalkArgs& a, int64_t gwarp, int64_t chunk) {
+    cursor = a.order ? 0 : gwarp * chunk;
+    end = a.order ? 0 : min(a.n, cursor + chunk);
+  }
+  __device__ __forceinline__ bool more(const WalkArgs& a) const {
+    return cursor < end || (a.order && end <= a.n);
+  }
+  // the track of the `rank`-th of `want` lanes, or -1 (warp-uniform but for
+  // rank; all lanes of the warp call it)
+  __device__ __forceinline__ int64_t take(const WalkArgs& a, int rank, int want) {
+    if (a.order && cursor >= end && end <= a.n) {
+      unsigned long long base = 0ull;
+      if ((threadIdx.x & 31) == 0) base = atomicAdd(a.work, 32ull);
+      base = __shfl_sync(0xffffffffu, base, 0);
+      cursor = (int64_t)base;
+      // (end stays past n once the order is used up, and no more is taken)
+      end = cursor < a.n ? min(a.n, cursor + 32) : a.n + 1;
+      if (cursor >= a.n) cursor = end;
+    }
+    const int64_t pos = cursor + rank;
+    cursor = min(end, cursor + want);
+    if (pos >= end || pos >= a.n) return -1;
+    if (!a.order) return pos;
+    const int64_t i = __ldg(&a.order[pos]);
+    return i >= 0 && i < a.n ? i : -1;  // (an entry out of range names no track)
+  }
+};
+
+// Persistent walk: a lane whose track has ended takes the warp's next one, so
+// a warp keeps all 32 lanes stepping until its tracks are used up (track
+// lengths are exponentially distributed, so one-track-per-lane would leave
+// most lanes idle behind the longest track of the warp).
 // SUM: the running length sum is wanted (WalkArgs::sum_out).
 template <int FO, bool MIXED, bool SUM>
 __global__ void __launch_bounds__(kBlock, 4) k_walk(WalkArgs a, int64_t chunk) {
   const int lane = threadIdx.x & 31;
   const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  // the warp's tracks: positions first + k * stride, k < count (a contiguous
-  // chunk, or with a length order every W-th track of it, longest first)
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int64_t first = a.order ? gwarp : gwarp * chunk;
-  const int64_t stride = a.order ? nwarps : 1;
-  const int64_t count = a.order ? (gwarp < a.n ? (a.n - gwarp + nwarps - 1) / nwarps : 0)
-                                : max((int64_t)0, min(a.n, first + chunk) - first);
-  int64_t cursor = 0;
-  const int64_t end = count;
+  WarpTracks list(a, gwarp, chunk);
   StepCnt cnt = {0, 0};
   unsigned long long tracks = 0;
   bool has = false;
@@ -432,14 +472,12 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(WalkArgs a, int64_t chunk) {
   double* ol = nullptr;
   while (true) {
     const unsigned need = __ballot_sync(0xffffffffu, !has);
-    if (need != 0u && cursor < end) {
+    if (need != 0u) {
+      unsigned lt;
+      asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
+      const int64_t cand = list.take(a, __popc(need & lt), __popc(need));
       if (!has) {
-        unsigned lt;
-        asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-        const int64_t kk = cursor + __popc(need & lt);
-        const int64_t pos = first + kk * stride;
-        const int64_t cand = kk < end ? (a.order ? (int64_t)__ldg(&a.order[pos]) : pos) : -1;
-        if (cand >= 0 && cand < a.n) {  // (an order entry out of range names no track)
+        if (cand >= 0) {
           i = cand;
           has = true;
           r = load3(a.org, i);
@@ -473,9 +511,11 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(WalkArgs a, int64_t chunk) {
           }
         }
       }
-      cursor += __popc(need);
     }
-    if (__ballot_sync(0xffffffffu, has) == 0u) break;
+    if (__ballot_sync(0xffffffffu, has) == 0u) {
+      if (list.more(a)) continue;
+      break;
+    }
     if (has) {
       bool done = !gt0(dist);  // while (distance > 0), mesh_manager_interface.cpp:117
       if (!done && k >= a.max_segs) {
@@ -485,24 +525,24 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(WalkArgs a, int64_t chunk) {
       if (!done) {
         cnt.steps++;
         double ex;
+        const TetRec T = load_rec(a, elem);
         const bool safe = sd.safe && in_range3(r);
-        const int f = next_face<FO, MIXED>(a, elem, r, u, sd, safe, &ex, cnt);
+        const int f = next_face<FO, MIXED>(a, T, r, u, sd, safe, &ex, cnt);
         int32_t nxt = -1;
         if (f < 0) {
           st = RAY_NO_EXIT_FACE;  // the reference would index adjacency with -1
         } else {
-          const int4 ad = __ldg(&a.adj[elem]);
-          nxt = f == 0 ? ad.x : (f == 1 ? ad.y : (f == 2 ? ad.z : ad.w));
+          nxt = sel4(T.adj, f);
         }
         ex = dlt(dist, ex) ? dist : ex;  // std::min(exit, distance)
         dist -= ex;
         if (SUM) sum = sum + ex;
         if (oe) {
-          oe[k] = __ldg(&a.elem_ids[elem]);
+          oe[k] = T.id;
           ol[k] = ex;
         }
         ++k;
-        r = walk_move(r, ex, u, safe);  // r += exit.second * u
+        r = add3(r, scl3(ex, u));  // r += exit.second * u
         if (nxt < -1 || nxt >= a.n_tets) {
           st = RAY_INVALID;  // corrupt adjacency: stop instead of reading out of range
           done = true;
@@ -543,13 +583,13 @@ __global__ void __launch_bounds__(kBlock) k_next(WalkArgs a) {
       st = RAY_INVALID;
     } else {
       cnt.steps++;
+      const TetRec T = load_rec(a, elem);
       const StepDir sd = step_dir(a, u);
-      const int f = next_face<FO, MIXED>(a, elem, r, u, sd, sd.safe && in_range3(r), &ex, cnt);
+      const int f = next_face<FO, MIXED>(a, T, r, u, sd, sd.safe && in_range3(r), &ex, cnt);
       if (f < 0) {
         st = RAY_NO_EXIT_FACE;
       } else {
-        const int4 ad = __ldg(&a.adj[elem]);
-        nxt = f == 0 ? ad.x : (f == 1 ? ad.y : (f == 2 ? ad.z : ad.w));
+        nxt = sel4(T.adj, f);
       }
     }
     a.next_out[i] = nxt;
@@ -641,15 +681,7 @@ __global__ void __launch_bounds__(kBlock) k_walk_q(WalkArgs a, int64_t chunk) {
   WalkQueue& Q = qs[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  // the warp's tracks: positions first + k * stride, k < count (a contiguous
-  // chunk, or with a length order every W-th track of it, longest first)
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int64_t first = a.order ? gwarp : gwarp * chunk;
-  const int64_t stride = a.order ? nwarps : 1;
-  const int64_t count = a.order ? (gwarp < a.n ? (a.n - gwarp + nwarps - 1) / nwarps : 0)
-                                : max((int64_t)0, min(a.n, first + chunk) - first);
-  int64_t cursor = 0;
-  const int64_t end = count;
+  WarpTracks list(a, gwarp, chunk);
   if (lane == 0) {
     Q.head = 0u;
     Q.tail = 0u;
@@ -677,14 +709,12 @@ __global__ void __launch_bounds__(kBlock) k_walk_q(WalkArgs a, int64_t chunk) {
   while (true) {
     // ---- refill lanes without a track from the warp's chunk ----
     const unsigned need = __ballot_sync(0xffffffffu, !has);
-    if (need != 0u && cursor < end) {
+    if (need != 0u) {
+      unsigned lt;
+      asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
+      const int64_t cand = list.take(a, __popc(need & lt), __popc(need));
       if (!has) {
-        unsigned lt;
-        asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-        const int64_t kk = cursor + __popc(need & lt);
-        const int64_t pos = first + kk * stride;
-        const int64_t cand = kk < end ? (a.order ? (int64_t)__ldg(&a.order[pos]) : pos) : -1;
-        if (cand >= 0 && cand < a.n) {  // (an order entry out of range names no track)
+        if (cand >= 0) {
           i = cand;
           has = true;
           in_step = false;
@@ -722,9 +752,11 @@ __global__ void __launch_bounds__(kBlock) k_walk_q(WalkArgs a, int64_t chunk) {
           }
         }
       }
-      cursor += __popc(need);
     }
-    if (__ballot_sync(0xffffffffu, has) == 0u) break;
+    if (__ballot_sync(0xffffffffu, has) == 0u) {
+      if (list.more(a)) continue;
+      break;
+    }
 
     // ---- start a step: FP32 filter, queue the faces it cannot reject ----
     unsigned escm = 0u;
@@ -749,7 +781,7 @@ __global__ void __launch_bounds__(kBlock) k_walk_q(WalkArgs a, int64_t chunk) {
       } else {
         cnt.steps++;
         in_step = true;
-        const int4 c = __ldg(&a.conn[elem]);
+        const int4 c = __ldg(a.rec + 4 * (int64_t)elem);
         ci[0] = c.x;
         ci[1] = c.y;
         ci[2] = c.z;
@@ -859,14 +891,14 @@ __global__ void __launch_bounds__(kBlock) k_walk_q(WalkArgs a, int64_t chunk) {
       if (bf < 0) {
         st = RAY_NO_EXIT_FACE;  // the reference would index adjacency with -1
       } else {
-        const int4 ad = __ldg(&a.adj[elem]);
+        const int4 ad = __ldg(a.rec + 4 * (int64_t)elem + 1);
         nxt = bf == 0 ? ad.x : (bf == 1 ? ad.y : (bf == 2 ? ad.z : ad.w));
       }
       ex = dlt(dist, ex) ? dist : ex;  // std::min(exit, distance)
       dist -= ex;
       if (a.sum_out) sum = sum + ex;
       if (oe) {
-        oe[k] = __ldg(&a.elem_ids[elem]);
+        oe[k] = __ldg(a.rec + 4 * (int64_t)elem + 3).z;
         ol[k] = ex;
       }
       ++k;
@@ -992,6 +1024,10 @@ cudaError_t launch_walk_s(const WalkArgs& a, cudaStream_t st) {
   if (blocks < 1) blocks = 1;
   const int64_t warps = blocks * (kBlock / 32);
   const int64_t chunk = (a.n + warps - 1) / warps;
+  if (a.order) {
+    const cudaError_t m = cudaMemsetAsync(a.work, 0, sizeof(*a.work), st);
+    if (m != cudaSuccess) return m;
+  }
   kern<<<(unsigned)blocks, kBlock, 0, st>>>(a, chunk);
   return cudaGetLastError();
 }
@@ -1063,14 +1099,13 @@ __global__ void __launch_bounds__(kBlock, 4) k_transport(TransportArgs t, int64_
 
   // moves the particle to the exit face and into the neighbour (:86-90);
   // returns true when it stops
-  auto exit_step = [&](double ex, int f) -> bool {
+  auto exit_step = [&](double ex, int f, const int32_t adj[4]) -> bool {
     if (f < 0) {
       st = RAY_NO_EXIT_FACE;  // exit = INFTY and c >= INFTY: no finite step exists
       return true;
     }
-    const int4 ad = __ldg(&a.adj[elem]);
-    const int32_t nxt = f == 0 ? ad.x : (f == 1 ? ad.y : (f == 2 ? ad.z : ad.w));
-    r = walk_move(r, ex, u, sd.safe && in_range3(r));
+    const int32_t nxt = sel4(adj, f);
+    r = add3(r, scl3(ex, u));
     dist += ex;
     if (t.tally) atomicAdd(&t.tally[elem], ex);
     if (nxt < -1 || nxt >= a.n_tets) {
@@ -1117,7 +1152,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_transport(TransportArgs t, int64_
       if (!done) {
         cnt.steps++;
         double ex;
-        const int f = next_face<FO, MIXED>(a, elem, r, u, sd, sd.safe && in_range3(r), &ex, cnt);
+        const TetRec T = load_rec(a, elem);
+        const int f = next_face<FO, MIXED>(a, T, r, u, sd, sd.safe && in_range3(r), &ex, cnt);
         // 1 - U of uniform53's U = k 2^-53 is (2^53 - k) 2^-53, exactly
         const unsigned long long U = (1ull << 53) - (splitmix_next(rs) >> 11);
         // Most events leave the tet: an FP32 logarithm with a certified
@@ -1131,7 +1167,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_transport(TransportArgs t, int64_
           leaves = dlt(ex, (double)lo);  // c >= lo > exit
         }
         if (leaves) {
-          done = exit_step(ex, f);
+          done = exit_step(ex, f, T.adj);
         } else {
           pend = true;  // the exact sample and the event run with the warp's batch
           pu = U;
@@ -1153,14 +1189,16 @@ __global__ void __launch_bounds__(kBlock, 4) k_transport(TransportArgs t, int64_
           const double c = -series_log((double)pu * 1.1102230246251565e-16) * t.mfp;
           if (dlt(c, pex)) {
             // collision inside the tet (:81-85)
-            r = walk_move(r, c, u, sd.safe && in_range3(r));
+            r = add3(r, scl3(c, u));
             dist += c;
             if (t.tally) atomicAdd(&t.tally[elem], c);
             u = sample_direction(rs);
             sd = step_dir(a, u);
             ++ev;
           } else {
-            done = exit_step(pex, pf);
+            const int4 ad = __ldg(a.rec + 4 * (int64_t)elem + 1);
+            const int32_t adj[4] = {ad.x, ad.y, ad.z, ad.w};
+            done = exit_step(pex, pf, adj);
           }
         }
       }
@@ -1214,13 +1252,6 @@ cudaError_t launch_transport(bool mixed, int face_order, const TransportArgs& a,
 }
 
 int64_t scan_scratch_entries(int64_t n) { return (n + kScanBlock - 1) / kScanBlock + 1; }
-
-namespace {
-__global__ void k_iota(int32_t* v, int64_t n) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < n) v[i] = (int32_t)i;
-}
-}  // namespace
 
 namespace {
 
@@ -1359,30 +1390,70 @@ cudaError_t build_edge_table(const double* xyz, const int4* conn, int64_t n_tets
   return cudaSuccess;
 }
 
-size_t walk_order_scratch_bytes(int64_t n) {
+namespace {
+__global__ void k_tet_records(const int4* __restrict__ conn, const int4* __restrict__ adj,
+                              const int32_t* __restrict__ tet_edge,
+                              const int32_t* __restrict__ ids, int64_t n, int4* __restrict__ rec) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  int32_t e[6] = {0, 0, 0, 0, 0, 0};
+  if (tet_edge)
+    for (int k = 0; k < 6; ++k) e[k] = tet_edge[6 * i + k];
+  rec[4 * i] = conn[i];
+  rec[4 * i + 1] = adj[i];
+  rec[4 * i + 2] = make_int4(e[0], e[1], e[2], e[3]);
+  rec[4 * i + 3] = make_int4(e[4], e[5], ids[i], 0);
+}
+}  // namespace
+
+cudaError_t build_tet_records(const int4* conn, const int4* adj, const int32_t* tet_edge,
+                              const int32_t* ids, int64_t n_tets, int4* rec, cudaStream_t st) {
+  if (n_tets <= 0) return cudaSuccess;
+  k_tet_records<<<(unsigned)((n_tets + 255) / 256), 256, 0, st>>>(conn, adj, tet_edge, ids, n_tets,
+                                                                  rec);
+  return cudaGetLastError();
+}
+
+namespace {
+// Sort keys of the length order: the length's FP32 exponent and leading 8
+// mantissa bits.  The order only groups tracks of about the same length, and
+// 16 bits take two radix passes where the 64 of the length took eight (1e6
+// tracks, two rounds: 215 -> 60 us).
+__global__ void k_length_keys(const double* __restrict__ dist, int64_t n,
+                              uint32_t* __restrict__ keys, int32_t* __restrict__ idx) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double d = dist[i];
+  keys[i] = gt0(d) && !nan_bits(d) ? __float_as_uint(f32_trunc(d)) >> 15 : 0u;
+  idx[i] = (int32_t)i;
+}
+constexpr int kLengthBits = 16;
+
+size_t length_sort_bytes(int64_t n) {
   size_t tmp = 0;
-  cub::DeviceRadixSort::SortPairsDescending(nullptr, tmp, (const double*)nullptr, (double*)nullptr,
-                                            (const int32_t*)nullptr, (int32_t*)nullptr, (int)n);
-  return ((tmp + 255) & ~(size_t)255) + ((sizeof(double) * n + 255) & ~(size_t)255) +
-         ((sizeof(int32_t) * n + 255) & ~(size_t)255);
+  cub::DeviceRadixSort::SortPairsDescending(nullptr, tmp, (const uint32_t*)nullptr,
+                                            (uint32_t*)nullptr, (const int32_t*)nullptr,
+                                            (int32_t*)nullptr, (int)n, 0, kLengthBits);
+  return (tmp + 255) & ~(size_t)255;
+}
+}  // namespace
+
+size_t walk_order_scratch_bytes(int64_t n) {
+  return length_sort_bytes(n) + 3 * ((sizeof(uint32_t) * n + 255) & ~(size_t)255);
 }
 
 cudaError_t walk_order(const double* dist, int64_t n, int32_t* order, void* scratch,
                        size_t scratch_bytes, cudaStream_t st) {
-  size_t tmp = 0;
-  cudaError_t e = cub::DeviceRadixSort::SortPairsDescending(
-      nullptr, tmp, (const double*)nullptr, (double*)nullptr, (const int32_t*)nullptr,
-      (int32_t*)nullptr, (int)n, 0, 64, st);
-  if (e != cudaSuccess) return e;
+  if (walk_order_scratch_bytes(n) > scratch_bytes) return cudaErrorInvalidValue;
+  size_t tmp = length_sort_bytes(n);
+  const size_t arr = (sizeof(uint32_t) * n + 255) & ~(size_t)255;
   char* p = (char*)scratch;
-  const size_t tmp_al = (tmp + 255) & ~(size_t)255;
-  double* keys_out = (double*)(p + tmp_al);
-  int32_t* idx = (int32_t*)(p + tmp_al + ((sizeof(double) * n + 255) & ~(size_t)255));
-  if (tmp_al + ((sizeof(double) * n + 255) & ~(size_t)255) + sizeof(int32_t) * n > scratch_bytes)
-    return cudaErrorInvalidValue;
-  k_iota<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(idx, n);
-  return cub::DeviceRadixSort::SortPairsDescending(p, tmp, dist, keys_out, idx, order, (int)n, 0,
-                                                   64, st);
+  uint32_t* keys = (uint32_t*)(p + tmp);
+  uint32_t* keys_out = (uint32_t*)(p + tmp + arr);
+  int32_t* idx = (int32_t*)(p + tmp + 2 * arr);
+  k_length_keys<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(dist, n, keys, idx);
+  return cub::DeviceRadixSort::SortPairsDescending(p, tmp, keys, keys_out, idx, order, (int)n, 0,
+                                                   kLengthBits, st);
 }
 
 cudaError_t scan_offsets(int64_t* offsets, int64_t n, int64_t* block_sums, cudaStream_t st) {

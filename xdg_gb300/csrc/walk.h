@@ -10,15 +10,15 @@ namespace xdgcu {
 struct WalkArgs {
   const double* xyz;     // 3 doubles per vertex
   const float4* xyz32;   // fl32 vertex, w = |v|_inf
-  const int4* conn;      // 4 vertex indices per tet
-  const int4* adj;       // 4 neighbour tets per tet (-1 boundary), face order
-  const int32_t* elem_ids;
+  // one 64-byte record per tet: 4 vertex indices; 4 neighbour tets (-1
+  // boundary), face order; 6 edge references for its local vertex pairs
+  // (0,1),(0,2),(0,3),(1,2),(1,3),(2,3) -- the edge index, bit 31 set when the
+  // pair's second vertex is the edge's lo (0 without an edge table); its mesh
+  // id; a pad
+  const int4* rec;
   // edge table of the mesh (may be null): 6 doubles per unique edge (e = hi -
-  // lo, then e x lo, lo/hi in first() order) and 6 entries per tet for its
-  // local vertex pairs (0,1),(0,2),(0,3),(1,2),(1,3),(2,3): the edge index,
-  // bit 31 set when the pair's second vertex is the edge's lo
+  // lo, then e x lo, lo/hi in first() order)
   const double* edge;
-  const int32_t* tet_edge;
   int32_t int_ok;        // every vertex coordinate is in_range() (imul64.cuh)
   int32_t n_tets;
   int32_t face[12];      // local face table
@@ -55,9 +55,10 @@ struct WalkArgs {
   int64_t capacity;
   // mixed walk: 1 = per-warp FP64 queue (k_walk_q), 0 = per-lane escalation
   int32_t walk_queue;
-  // optional: track indices by decreasing length; the kernels then deal them
-  // round-robin to warps, longest first, so warps finish on short tracks
+  // optional: track indices by decreasing length; the warps then take them 32
+  // at a time, longest first, from the work counter (zero at launch)
   const int32_t* order;
+  unsigned long long* work;
   int32_t flush_wait;  // queue: lanes waiting that force a partial FP64 round
 };
 
@@ -89,13 +90,18 @@ cudaError_t launch_transport(bool mixed, int face_order, const TransportArgs& a,
 int64_t scan_scratch_entries(int64_t n);
 cudaError_t scan_offsets(int64_t* offsets, int64_t n, int64_t* block_sums, cudaStream_t st);
 
-// Length order of n tracks (n < 2^31): order[k] = index of the k-th longest.
+// Length order of n tracks (n < 2^31): order[k] = index of the k-th longest,
+// lengths compared to 8 bits of their significand.
 // scratch holds walk_order_scratch_bytes(n) bytes.
 size_t walk_order_scratch_bytes(int64_t n);
 cudaError_t walk_order(const double* dist, int64_t n, int32_t* order, void* scratch,
                        size_t scratch_bytes, cudaStream_t st);
 
-// Builds the edge table of a tet mesh (WalkArgs::edge / tet_edge) on the
+// The records of WalkArgs::rec (tet_edge: build_edge_table's, or null).
+cudaError_t build_tet_records(const int4* conn, const int4* adj, const int32_t* tet_edge,
+                              const int32_t* ids, int64_t n_tets, int4* rec, cudaStream_t st);
+
+// Builds the edge table of a tet mesh (WalkArgs::edge, edge references) on the
 // device: sorts the 6 vertex pairs of every tet, numbers the unique ones and
 // evaluates each edge's e and e x lo once, with plucker.h:45-62's operations.
 // *edge and *tet_edge are cudaMalloc'ed (the caller frees them).  Returns
