@@ -30,6 +30,7 @@
 #include "../../include/xdgcu.h"
 #include "bvh.h"
 #include "cbound.h"
+#include "cobb.h"
 #include "imul64.cuh"
 #include "queries.h"
 #include "segments.h"
@@ -49,6 +50,7 @@ struct SurfaceRec {
   int32_t rev_tree = -1;
   int32_t bc = 0;  // boundary condition for the particle loop (xdgcu_set_surface_boundary)
   double bump = 0.0;
+  bool int_ok = true;  // every vertex coordinate is in_range_of<60>() (imul64.cuh)
 };
 
 struct TreeHost {
@@ -59,6 +61,7 @@ struct TreeHost {
   DevMem<float4> prim32;
   DevMem<double> prim64;
   DevMem<int32_t> prim_ref;
+  DevMem<float4> obb;  // TreeDev::obb
   int32_t n_nodes = 0;
   int32_t depth = 0;
   TreeDev dev{};
@@ -224,6 +227,162 @@ __global__ void k_tri_cbound(const double* __restrict__ tri_xyz, int64_t n,
   float r[16];
   tri_cbound(tri_xyz + 9 * g, r);
   for (int k = 0; k < 4; ++k) out[4 * g + k] = make_float4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
+}
+
+// The oriented boxes of closest (TreeDev::obb, cobb.h), one group of threads
+// per child slot: eight lanes for ranges of up to kObbSmall primitives (larger
+// ones go to the list `big`), a block for the listed ones.  Most slots hold a
+// few triangles, and the FP64 unit takes as long for one lane as for 32, so
+// four slots share a warp and only the slabs are evaluated in FP64 (the axes,
+// which only decide how tight they are, in FP32; extremes are compared on the
+// integer pipes).
+constexpr int kObbSmall = 256, kObbBlock = 512, kObbLanes = 8;
+
+template <bool BIG>
+struct ObbGroup {
+  unsigned long long* sm;  // BIG: one slot per warp
+  template <typename T, typename Op>
+  __device__ T all(T v, Op op) {
+    for (int off = (BIG ? 32 : kObbLanes) / 2; off > 0; off >>= 1)
+      v = op(v, __shfl_xor_sync(0xffffffffu, v, off));
+    if (BIG) {
+      T* s = reinterpret_cast<T*>(sm);
+      __syncthreads();
+      if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
+      __syncthreads();
+      v = s[0];
+      for (int w = 1; w < kObbBlock / 32; ++w) v = op(v, s[w]);
+    }
+    return v;
+  }
+  __device__ float sum(float v) {
+    return all(v, [](float a, float b) { return a + b; });
+  }
+  __device__ double least(double v) {
+    return all(v, [](double a, double b) { return dlt(b, a) ? b : a; });
+  }
+  __device__ double most(double v) {
+    return all(v, [](double a, double b) { return dlt(a, b) ? b : a; });
+  }
+};
+
+// (a slot without primitives, n = 0, takes part in the group's reductions only)
+template <bool BIG>
+__device__ void obb_slot(ObbGroup<BIG> G, const double* __restrict__ prim64, int2 range, int64_t slot,
+                         float4* __restrict__ obb, float max_abs) {
+  const int stride = BIG ? kObbBlock : kObbLanes;
+  const int me = BIG ? threadIdx.x : (threadIdx.x & (kObbLanes - 1));
+  const double* v0 = prim64 + kPrim64Stride * (int64_t)range.x;
+  float org[3] = {0.0f, 0.0f, 0.0f};
+  if (range.y > 0)
+    for (int k = 0; k < 3; ++k) org[k] = f32_trunc(v0[k]);
+  auto local = [&](const double* v, float w[9]) {
+    for (int k = 0; k < 9; ++k) w[k] = f32_trunc(v[k]) - org[k % 3];
+  };
+  float ns[3] = {0, 0, 0}, area = 0.0f, vm[3] = {0, 0, 0};
+  for (int j = me; j < range.y; j += stride) {
+    float w[9];
+    local(v0 + kPrim64Stride * (int64_t)j, w);
+    const float a[3] = {w[3] - w[0], w[4] - w[1], w[5] - w[2]};
+    const float b[3] = {w[6] - w[0], w[7] - w[1], w[8] - w[2]};
+    const float n[3] = {a[1] * b[2] - a[2] * b[1], a[2] * b[0] - a[0] * b[2],
+                        a[0] * b[1] - a[1] * b[0]};
+    for (int k = 0; k < 3; ++k) ns[k] += n[k];
+    area += sqrtf(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+    for (int k = 0; k < 9; ++k) vm[k % 3] += w[k];
+  }
+  for (int k = 0; k < 3; ++k) {
+    ns[k] = G.sum(ns[k]);
+    vm[k] = G.sum(vm[k]) / (3.0f * max(range.y, 1));
+  }
+  area = G.sum(area);
+  float row[3][3];
+  obb_axes(ns, area, row);
+  float sxx = 0.0f, sxy = 0.0f, syy = 0.0f;
+  for (int j = me; j < range.y; j += stride) {
+    float w[9];
+    local(v0 + kPrim64Stride * (int64_t)j, w);
+    for (int k = 0; k < 9; k += 3) {
+      float x = 0.0f, y = 0.0f;
+      for (int i = 0; i < 3; ++i) {
+        x += (w[k + i] - vm[i]) * row[1][i];
+        y += (w[k + i] - vm[i]) * row[2][i];
+      }
+      sxx += x * x;
+      sxy += x * y;
+      syy += y * y;
+    }
+  }
+  sxx = G.sum(sxx);
+  sxy = G.sum(sxy);
+  syy = G.sum(syy);
+  obb_turn(sxx, sxy, syy, row[1], row[2]);
+  float a[3][3];
+  obb_rows32(row, a);
+  double lo[3], hi[3];
+  for (int i = 0; i < 3; ++i) {
+    lo[i] = INFTY;
+    hi[i] = -INFTY;
+  }
+  for (int j = me; j < range.y; j += stride) {
+    const double* v = v0 + kPrim64Stride * (int64_t)j;
+    for (int k = 0; k < 9; k += 3)
+      for (int i = 0; i < 3; ++i) {
+        const double x = obb_dot(a[i], v + k);
+        lo[i] = dlt(x, lo[i]) ? x : lo[i];
+        hi[i] = dlt(hi[i], x) ? x : hi[i];
+      }
+  }
+  float* out = reinterpret_cast<float*>(obb + kObbRec * (slot / kWidth)) + slot % kWidth;
+  for (int i = 0; i < 3; ++i) {
+    lo[i] = G.least(lo[i]);
+    hi[i] = G.most(hi[i]);
+    if (me == i && range.y > 0) {
+      float d = 0.0f, h = 0.0f;
+      obb_slab(lo[i], hi[i], (double)max_abs, &d, &h);
+      for (int k = 0; k < 3; ++k) out[4 * (1 + 5 * i + k)] = a[i][k];
+      out[4 * (1 + 5 * i + 3)] = d;
+      out[4 * (1 + 5 * i + 4)] = h;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(128) k_obb_small(const double* __restrict__ prim64,
+                                                   const Node32* __restrict__ n32,
+                                                   const int2* __restrict__ ranges, int64_t slots,
+                                                   float max_abs, float4* __restrict__ obb,
+                                                   int64_t* __restrict__ big,
+                                                   unsigned long long* __restrict__ n_big) {
+  const int64_t slot = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kObbLanes;
+  const int me = threadIdx.x & (kObbLanes - 1);
+  int2 range = make_int2(0, 0);
+  if (slot < slots) {
+    const int4 c = n32[slot / kWidth].child;
+    const int k = (int)(slot % kWidth);
+    float* rec = reinterpret_cast<float*>(obb + kObbRec * (slot / kWidth));
+    if (me == 0) rec[k] = __int_as_float(k == 0 ? c.x : (k == 1 ? c.y : (k == 2 ? c.z : c.w)));
+    range = ranges[slot];
+    if (range.y <= 0) {
+      for (int q = me; q < 15; q += kObbLanes) rec[4 * (1 + q) + k] = 0.0f;
+      range = make_int2(0, 0);
+    } else if (range.y > kObbSmall) {
+      if (me == 0) big[atomicAdd(n_big, 1ull)] = slot;
+      range = make_int2(0, 0);
+    }
+  }
+  // (all lanes: the reductions are warp-wide)
+  obb_slot<false>(ObbGroup<false>{nullptr}, prim64, range, slot, obb, max_abs);
+}
+
+__global__ void __launch_bounds__(kObbBlock) k_obb_big(const double* __restrict__ prim64,
+                                                       const int2* __restrict__ ranges,
+                                                       const int64_t* __restrict__ big,
+                                                       const unsigned long long* __restrict__ n_big,
+                                                       float max_abs, float4* __restrict__ obb) {
+  __shared__ unsigned long long sm[kObbBlock / 32];
+  const unsigned long long m = *n_big;
+  for (unsigned long long b = blockIdx.x; b < m; b += gridDim.x)
+    obb_slot<true>(ObbGroup<true>{sm}, prim64, ranges[big[b]], big[b], obb, max_abs);
 }
 
 __global__ void k_tet_boxes(const double* __restrict__ xyz, const int4* __restrict__ conn,
@@ -545,6 +704,7 @@ void fill_dev(TreeHost& t, const BuiltTree& b, double min_bump) {
   TreeDev& d = t.dev;
   d.n32 = b.n32;
   d.n64 = b.n64;
+  d.obb = t.obb.p;
   d.prim32 = t.prim32.p;
   d.prim64 = t.prim64.p;
   d.prim_ref = t.prim_ref.p;
@@ -586,7 +746,7 @@ int build_surface_bvh(xdgcu_ctx* c, TreeHost& t, const std::vector<int32_t>& tri
   BuiltTree b;
   const BvhCost cost{1.0, c->bvh_prim_cost * 1e-3};
   API_CUDA(build_wide_bvh(d_box.p, n, c->leaf_max, c->node_width, c->bvh_sah ? &cost : nullptr,
-                          st, &b),
+                          st, &b, true),
            "bvh build");
   API_CUDA(t.prim32.alloc(3 * (int64_t)std::max(1, n)), "alloc prims");
   API_CUDA(t.prim64.alloc(kPrim64Stride * (int64_t)std::max(1, n)), "alloc prims");
@@ -596,10 +756,35 @@ int build_surface_bvh(xdgcu_ctx* c, TreeHost& t, const std::vector<int32_t>& tri
                                           t.prim64.p, t.prim_ref.p);
     API_CUDA(cudaGetLastError(), "gather");
   }
+  t.obb.reset();
+  if (b.ranges && b.n_nodes > 0) {
+    const int64_t recs = (int64_t)b.n_nodes * (b.width / kWidth), slots = recs * kWidth;
+    // a slot of more than kObbSmall primitives: at most one per that many
+    // primitives on each level of the tree
+    DevMem<int64_t> big(std::min<int64_t>(slots, ((int64_t)n / kObbSmall + 1) * (b.depth + 1)));
+    DevMem<unsigned long long> n_big(1);
+    API_CUDA(t.obb.alloc(kObbRec * recs), "alloc closest boxes");
+    API_CUDA(big.alloc(), "alloc");
+    API_CUDA(n_big.alloc(), "alloc");
+    API_CUDA(cudaMemsetAsync(n_big.p, 0, sizeof(unsigned long long), st), "memset");
+    double m = 0.0;
+    for (int k = 0; k < 6; ++k) m = std::max(m, std::fabs(b.bounds[k]));
+    const float max_abs = std::nextafter((float)m, INFINITY);
+    k_obb_small<<<grid(kObbLanes * slots, 128), 128, 0, st>>>(t.prim64.p, b.n32, b.ranges, slots,
+                                                               max_abs, t.obb.p, big.p, n_big.p);
+    k_obb_big<<<2 * device_sm_count(), kObbBlock, 0, st>>>(t.prim64.p, b.ranges, big.p, n_big.p,
+                                                          max_abs, t.obb.p);
+    API_CUDA(cudaGetLastError(), "closest boxes");
+    API_CUDA(cudaStreamSynchronize(st), "closest boxes");
+  }
+  if (b.ranges) cudaFree(b.ranges);
   API_CUDA(cudaStreamSynchronize(st), "build sync");
   if (b.order) cudaFree(b.order);
   t.prim_ref.n = n;
   fill_dev(t, b, n > 0 ? min_bump : 1e-3);
+  t.dev.int_ok = 1;
+  for (int32_t m : t.members)
+    if (!c->surfs[m].int_ok) t.dev.int_ok = 0;
   return XDGCU_OK;
 }
 
@@ -1353,6 +1538,7 @@ int xdgcu_register_surface(xdgcu_ctx* c, int32_t surface_id, int64_t n_faces, co
   r.id = surface_id;
   r.first = (int64_t)c->h_tri_face.size();
   r.count = n_faces;
+  for (int64_t i = 0; i < 9 * n_faces; ++i) r.int_ok = r.int_ok && in_range_of<60>(tri_xyz[i]);
   const int32_t sidx = (int32_t)c->surfs.size();
   c->surf_index[surface_id] = sidx;
   c->surfs.push_back(r);

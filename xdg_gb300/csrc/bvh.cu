@@ -193,6 +193,7 @@ struct CollapseArgs {
   Node64* n64;
   int32_t* node_counter;
   int32_t* out_count;
+  int2* ranges;  // may be null
 };
 
 __device__ __forceinline__ double half_area(const double* b) {
@@ -397,6 +398,9 @@ __global__ void k_collapse(CollapseArgs A, const int2* __restrict__ in, int32_t 
         f32[2 * a + 1][kk] = __double2float_ru(bx[3 + a]);
       }
       const int32_t cc = count_of(c);
+      if (A.ranges)
+        A.ranges[((int64_t)w * (W / kWidth) + rec) * kWidth + kk] =
+            make_int2(is_inner(c) ? A.first[c] : c - (n - 1), cc);
       const bool leaf = use_sah ? (!is_inner(c) || sah.dec[(int64_t)c * W] == 0)
                                 : (!is_inner(c) || cc <= A.leaf_max);
       if (leaf) {
@@ -416,6 +420,8 @@ __global__ void k_collapse(CollapseArgs A, const int2* __restrict__ in, int32_t 
         f32[2 * a + 1][kk] = -INFINITY;
       }
       refs[kk] = CHILD_EMPTY;
+      if (A.ranges)
+        A.ranges[((int64_t)w * (W / kWidth) + rec) * kWidth + kk] = make_int2(0, 0);
     }
   }
   n32.child = make_int4(refs[0], refs[1], refs[2], refs[3]);
@@ -434,12 +440,14 @@ __global__ void k_collapse(CollapseArgs A, const int2* __restrict__ in, int32_t 
   } while (0)
 
 cudaError_t build_wide_bvh(const double* d_boxes, int32_t n, int32_t leaf_max, int32_t width,
-                           const BvhCost* sah_cost, cudaStream_t st, BuiltTree* out) {
+                           const BvhCost* sah_cost, cudaStream_t st, BuiltTree* out,
+                           bool want_ranges) {
   if (width != 4 && width != 8) return cudaErrorInvalidValue;
   out->width = width;
   out->n32 = nullptr;
   out->n64 = nullptr;
   out->order = nullptr;
+  out->ranges = nullptr;
   out->n_nodes = 0;
   out->depth = 0;
   out->root = CHILD_EMPTY;
@@ -554,6 +562,7 @@ cudaError_t build_wide_bvh(const double* d_boxes, int32_t n, int32_t leaf_max, i
   const int64_t recs = (int64_t)cap * (width / kWidth);
   BVH_CHECK(cudaMalloc(&out->n32, sizeof(Node32) * recs));
   BVH_CHECK(cudaMalloc(&out->n64, sizeof(Node64) * recs));
+  if (want_ranges) BVH_CHECK(cudaMalloc(&out->ranges, sizeof(int2) * recs * kWidth));
   DevMem<int2> qa(cap), qb(cap);
   DevMem<int32_t> counters(2);  // [0] node counter, [1] out count
   BVH_CHECK(qa.alloc());
@@ -564,7 +573,7 @@ cudaError_t build_wide_bvh(const double* d_boxes, int32_t n, int32_t leaf_max, i
   BVH_CHECK(cudaMemcpyAsync(qa.p, &root_item, sizeof root_item, cudaMemcpyHostToDevice, st));
   BVH_CHECK(cudaMemcpyAsync(counters.p, hc, sizeof hc, cudaMemcpyHostToDevice, st));
   CollapseArgs A{left.p, right.p, first.p, last.p, nbox.p, n, leaf_max,
-                 out->n32, out->n64, counters.p, counters.p + 1};
+                 out->n32, out->n64, counters.p, counters.p + 1, out->ranges};
   int32_t n_in = 1;
   int depth = 0;
   int2* qin = qa.p;

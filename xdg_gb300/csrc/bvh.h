@@ -52,7 +52,7 @@ struct DevMem {
   size_t bytes() const { return sizeof(T) * (size_t)n; }
 };
 
-// Result of build_wide_bvh.  n32/n64/order are cudaMalloc'ed and owned by the
+// Result of build_wide_bvh.  n32/n64/order/ranges are cudaMalloc'ed and owned by the
 // caller afterwards.  order[j] = input primitive index at leaf position j.
 struct BuiltTree {
   Node32* n32;
@@ -62,6 +62,8 @@ struct BuiltTree {
   int32_t depth;
   int32_t root;
   int32_t width;     // children per node: 4 (one record) or 8 (two records)
+  int2* ranges;      // per record and slot: the child's first leaf position and
+                     // its number of primitives (when asked for, else null)
   double bounds[6];  // union of the primitive boxes
 };
 
@@ -76,6 +78,7 @@ struct BvhCost {
 // sah_cost: collapse by the SAH (bvh.cu, step 6a), or nullptr for the greedy
 // largest-area collapse (6b).
 cudaError_t build_wide_bvh(const double* d_boxes, int32_t n, int32_t leaf_max, int32_t width,
-                           const BvhCost* sah_cost, cudaStream_t st, BuiltTree* out);
+                           const BvhCost* sah_cost, cudaStream_t st, BuiltTree* out,
+                           bool want_ranges = false);
 
 }  // namespace xdgcu

@@ -100,11 +100,13 @@ XDG_HD double mul_int(double a, double b) {
   return from_words(zero ? 0u : (uint32_t)r, zero ? sign : (uint32_t)(r >> 32));
 }
 
-// x is +-0 or 2^-150 <= |x| < 2^150
-XDG_HD bool in_range(double x) {
+// x is +-0 or 2^-P <= |x| < 2^P
+template <int P>
+XDG_HD bool in_range_of(double x) {
   const W64 w = words(x);
   const uint32_t h = w.hi & 0x7fffffffu;
-  return h - ((1023u - 150u) << 20) < (300u << 20) || (h | w.lo) == 0u;
+  return h - ((1023u - P) << 20) < ((2u * P) << 20) || (h | w.lo) == 0u;
 }
+XDG_HD bool in_range(double x) { return in_range_of<150>(x); }
 
 }  // namespace xdgcu

@@ -61,9 +61,15 @@ enum TreeKind : int32_t { TREE_SURFACE = 0, TREE_ELEMENT = 1 };
 //                  prim64 = 10 doubles per triangle (v0, v1, v2, pad)
 //                  prim_ref = global triangle index
 //   element trees: prim64 = 12 doubles per tet (v0..v3), prim_ref = tet index
+// Surface trees also hold, per 4-wide record, 16 float4 for closest (cobb.h):
+// the child references, then for each of three axes the four children's row
+// x, y, z, middle d and half width h.
+constexpr int kObbRec = 16;
+
 struct TreeDev {
   const Node32* n32;
   const Node64* n64;
+  const float4* obb;  // surface trees with inner nodes, else null
   const float4* prim32;
   const double* prim64;
   const int32_t* prim_ref;
@@ -75,6 +81,8 @@ struct TreeDev {
   float max_abs;     // max |coordinate| over the tree's (bumped) bounds
   int32_t kind;
   int32_t width;     // 4 or 8 children per node; node k = records k*width/4 ..
+  int32_t int_ok;    // surface trees: every vertex coordinate is 0 or 2^-60 .. 2^60
+                     // in magnitude (closest_dist_i)
 };
 
 constexpr int kPrim64Stride = 10;  // doubles per triangle in prim64

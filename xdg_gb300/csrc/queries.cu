@@ -10,6 +10,7 @@
 // reference's FP64 formulas from geom.cuh, so results are bit-identical.
 #include <algorithm>
 
+#include "imul64.cuh"
 #include "queries.h"
 #include "traverse.cuh"
 
@@ -38,83 +39,87 @@ __device__ __forceinline__ int64_t point_index(const PointArgs& a) {
 constexpr int kCand = 8;
 
 // The children of record `rec` of inner node `ref` that may hold a facet no
-// farther than `best`: their references in cr and lower bounds of the
-// point's distance to their boxes in ck (FP32, rounded down; 0 where FP32
-// cannot prune), nearest first.  Returns their number.
+// farther than the best: their references in cr and lower bounds of the
+// point's distance to them in ck (FP32; 0 where FP32 cannot prune), nearest
+// first.  Returns their number.
+//
+// Mixed: the children's oriented boxes (TreeDev::obb, cobb.h) against
+// `bestf`, the best distance rounded up.  The FP32 products (p rounded, three
+// FMAs a row, |a| < 1) are within 7 u (|p| + M) of a . p - d, so the bound less
+// cmargin = 48 u (|p| + M) undershoots the distance (M = max_abs, as in
+// closest_lower_of).  The boxes follow the surface where axis-aligned ones
+// stick out by a triangle's tilt: on the nested spheres the node visits went
+// from 60.5 to 35.1, the triangles bounded from 78.5 to 18.2 and the exact
+// tests from 12.0 to 4.5 a point, and 1e6 points from 16.0 to 5.3 ms (the
+// node's 256 bytes against 112 included).
+// All-FP64: the distance to the FP64 boxes, computed in FP64, its lower bound
+// in FP32 against `bestf`.
 template <bool MIXED>
 __device__ __forceinline__ int closest_children(const TreeDev& T, int32_t ref, int rec, d3 p,
-                                                float px, float py, float pz, float pabs,
-                                                bool f32ok, double best, int32_t cr[4],
+                                                float px, float py, float pz, float cmargin,
+                                                bool f32ok, float bestf, int32_t cr[4],
                                                 float ck[4]) {
   const int nrec = T.width / kWidth;
   int nhit = 0;
   if (MIXED) {
-    const Node32* np = T.n32 + (int64_t)ref * nrec + rec;
-    const float4 lx = __ldg(&np->lox), hx = __ldg(&np->hix), ly = __ldg(&np->loy),
-                 hy = __ldg(&np->hiy), lz = __ldg(&np->loz), hz = __ldg(&np->hiz);
-    const int4 c = __ldg(&np->child);
-    const float la[3][4] = {{lx.x, lx.y, lx.z, lx.w}, {ly.x, ly.y, ly.z, ly.w},
-                            {lz.x, lz.y, lz.z, lz.w}};
-    const float ha[3][4] = {{hx.x, hx.y, hx.z, hx.w}, {hy.x, hy.y, hy.z, hy.w},
-                            {hz.x, hz.y, hz.z, hz.w}};
-    const float pa[3] = {px, py, pz};
+    const float4* R = T.obb + kObbRec * ((int64_t)ref * nrec + rec);
+    const int4 c = __ldg(reinterpret_cast<const int4*>(R));
     const int32_t ca[4] = {c.x, c.y, c.z, c.w};
-    // prune only when the FP32 distance, shrunk by its error bound,
-    // exceeds the current best (rounded up to float)
-    const float bestf = __double2float_ru(best);
-    float key[4];
+    float s2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const float4 ax = __ldg(R + 1 + 5 * i), ay = __ldg(R + 2 + 5 * i), az = __ldg(R + 3 + 5 * i),
+                   d = __ldg(R + 4 + 5 * i), h = __ldg(R + 5 + 5 * i);
+      const float axa[4] = {ax.x, ax.y, ax.z, ax.w}, aya[4] = {ay.x, ay.y, ay.z, ay.w};
+      const float aza[4] = {az.x, az.y, az.z, az.w}, da[4] = {d.x, d.y, d.z, d.w};
+      const float ha[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float s = __fmaf_rn(axa[k], px, __fmaf_rn(aya[k], py, __fmaf_rn(aza[k], pz, -da[k])));
+        const float e = fmaxf(fabsf(s) - ha[k], 0.0f);
+        s2[k] = __fmaf_rn(e, e, s2[k]);
+      }
+    }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      float s2 = 0.0f;
-      bool empty = false;
-#pragma unroll
-      for (int ax = 0; ax < 3; ++ax) {
-        empty |= !(la[ax][k] <= ha[ax][k]);
-        const float e = fmaxf(fmaxf(la[ax][k] - pa[ax], pa[ax] - ha[ax][k]), 0.0f);
-        s2 += e * e;
-      }
-      const float dist = sqrtf(s2);
-      const float lb = dist * (1.0f - 8.0f * kU32) - 4.0f * kU32 * pabs;
+      const float lb = __fsqrt_rn(s2[k]) * (1.0f - 8.0f * kU32) - cmargin;
       // the key is the lower bound itself (0 where FP32 cannot prune)
-      key[k] = (!empty && (lb <= bestf || !f32ok)) ? (f32ok ? fmaxf(lb, 0.0f) : 0.0f) : INFINITY;
+      ck[k] = (ca[k] != CHILD_EMPTY && (lb <= bestf || !f32ok)) ? (f32ok ? fmaxf(lb, 0.0f) : 0.0f)
+                                                                : INFINITY;
       cr[k] = ca[k];
     }
-    sort4(key, cr);
+    sort4(ck, cr);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      nhit += key[k] < INFINITY ? 1 : 0;
-      ck[k] = key[k];
-    }
+    for (int k = 0; k < 4; ++k) nhit += ck[k] < INFINITY ? 1 : 0;
   } else {
     const Node64* np = T.n64 + (int64_t)ref * nrec + rec;
     const int4 c = __ldg(&np->child);
     const int32_t ca[4] = {c.x, c.y, c.z, c.w};
-    double key[4];
     const double pa[3] = {p.x, p.y, p.z};
     const double* lo[3] = {np->lox, np->loy, np->loz};
     const double* hi[3] = {np->hix, np->hiy, np->hiz};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       double s2 = 0.0;
-      bool empty = false;
 #pragma unroll
       for (int ax = 0; ax < 3; ++ax) {
+        // the distance beyond the nearer face: one difference, the sides
+        // compared on the integer pipes (a difference is >= 0 or the side is
+        // not the one beyond which p lies, and a zero adds nothing)
         const double l = __ldg(lo[ax] + k), u = __ldg(hi[ax] + k);
-        empty |= !(l <= u);
-        const double e = fmax(fmax(l - pa[ax], pa[ax] - u), 0.0);
+        const bool below = dlt(pa[ax], l), above = dlt(u, pa[ax]);
+        const double e = (below ? l : pa[ax]) - (below || !above ? pa[ax] : u);
         s2 += e * e;
       }
-      const double dist = sqrt(s2);
-      key[k] = (!empty && dist * (1.0 - 1e-12) <= best) ? dist : INFINITY;
+      // a lower bound of the distance in FP32: its square truncated (and cut
+      // at the largest float), less the root's rounding and that of s2
+      const float lb = __fsqrt_rn(fminf(f32_trunc(s2), 3.402823466e38f)) * (1.0f - 8.0f * kU32);
+      ck[k] = ca[k] != CHILD_EMPTY && lb <= bestf ? lb : INFINITY;
       cr[k] = ca[k];
     }
-    sort4d(key, cr);
+    sort4(ck, cr);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      nhit += key[k] < INFINITY ? 1 : 0;
-      // rounded down: a lower bound of dist * (1 - 1e-12)
-      ck[k] = key[k] < INFINITY ? __double2float_rd(key[k] * (1.0 - 1e-12)) : INFINITY;
-    }
+    for (int k = 0; k < 4; ++k) nhit += ck[k] < INFINITY ? 1 : 0;
   }
   return nhit;
 }
@@ -256,6 +261,141 @@ __device__ __forceinline__ RecordBounds closest_record_bounds(const PlaneDists& 
   return r;
 }
 
+// The distance of closest.cpp:54-183's point on triangle (v0, v1, v2) from p
+// (closest64, then dist64), for coordinates that are zero or of magnitude
+// 2^-60 .. 2^60: the same operations on the same operands, with the products
+// and the comparisons on the integer pipes (imul64.cuh).  The regions differ
+// only in which quotient they take and which vectors it scales, so the lanes
+// of a warp select the operands and then run one quotient and one
+//   (A + x B) + y C
+// together; as branches, each region's sums, products and divisions held the
+// FP64 unit for the whole warp.  (Adding +-0, and A = 0 or x = 0, changes a
+// result's bits at most in the sign of a zero, which the distance does not
+// see.)  A test then takes about 56 FP64 unit instructions, a quotient and a
+// root among them, whatever the regions of the warp's lanes.
+// Every product is normal or zero: with |coordinate| in that range the edges
+// are zero or above 2^-113, their dot products above 2^-278 and the region
+// variables above 2^-608; region six's weights may overflow for degenerate
+// triangles, and the point's offsets may leave the range, so those take the
+// FP64 unit's functions, which are called to stay behind a real branch.
+__device__ __noinline__ double closest_dist_hw(const double* v, d3 p) {
+  d3 v0, v1, v2;
+  load_tri64(v, v0, v1, v2);
+  return dist64(closest64(v0, v1, v2, p), p);
+}
+
+__device__ __forceinline__ bool range60(d3 a) {
+  return in_range_of<60>(a.x) && in_range_of<60>(a.y) && in_range_of<60>(a.z);
+}
+
+__device__ __forceinline__ double closest_dist_i(const double* tri, d3 p) {
+  auto dot_i = [](d3 a, d3 b) {
+    return mul_int(a.x, b.x) + mul_int(a.y, b.y) + mul_int(a.z, b.z);
+  };
+  auto sel = [](bool c, d3 a, d3 b) { return mk3(c ? a.x : b.x, c ? a.y : b.y, c ? a.z : b.z); };
+  d3 v0, v1, v2;
+  load_tri64(tri, v0, v1, v2);
+  const d3 sv = sub3(v1, v0), tv = sub3(v2, v0), pv = sub3(v0, p);
+  const double ss = dot_i(sv, sv), st = dot_i(sv, tv), tt = dot_i(tv, tv);
+  const double sp = dot_i(sv, pv), tp = dot_i(tv, pv);
+  const double det = mul_int(ss, tt) - mul_int(st, st);
+  const double s = mul_int(st, tp) - mul_int(tt, sp);
+  const double t = mul_int(st, sp) - mul_int(ss, tp);
+  const bool sn = lt0(s), tn = lt0(t), in = dlt(s + t, det);
+  // closest.cpp:6-28
+  const int region = in ? (sn ? (tn ? 4 : 3) : (tn ? 5 : 0)) : (sn ? 2 : (tn ? 6 : 1));
+  // The candidates' scalars, each by its region's operations:
+  //   1: num = ((tt + tp) - st) - sp        2: num = (tt + tp) - (st + sp)
+  //   6: num = (st + tp) - (ss + sp)        den = (ss - 2 st) + tt, 6: (tt - 2 st) + ss
+  const bool r1 = region == 1, r6 = region == 6;
+  const double X = (r6 ? st : tt) + tp;
+  const double Y = (r6 ? ss : st) + sp;
+  double num = X - (r1 ? st : Y);
+  num = num - (r1 ? sp : 0.0);
+  const double den = ((r6 ? tt : ss) - (st + st)) + (r6 ? ss : tt);
+  const double zero = 0.0;
+  // what the region returns: a vertex (kind 0), v0 - (sp / ss) sv (1),
+  // v0 - (tp / tt) tv (2), q v1 + (1 - q) v2 (3), (1 - q) v1 + q v2 (4), or
+  // the interior point (5)
+  int kind = 0, vertex = 0;
+  const bool sp_neg = lt0(sp), tp_neg = lt0(tp);
+  const double msp = -sp, mtp = -tp;
+  if (region == 0) {
+    kind = 5;
+  } else if (r1) {
+    if (!gt0(num)) vertex = 2;
+    else if (!dlt(num, den)) vertex = 1;
+    else kind = 3;
+  } else if (region == 2) {
+    if (dlt(Y, X)) {  // t > s
+      if (dlt(den, num)) vertex = 1;
+      else kind = 3;
+    } else if (!gt0(X)) {
+      vertex = 2;
+    } else if (tp_neg) {
+      kind = 2;
+    }
+  } else if (region == 3) {
+    if (tp_neg) {
+      if (!dlt(mtp, tt)) vertex = 2;
+      else kind = 2;
+    }
+  } else if (region == 4) {
+    if (sp_neg) {
+      if (dlt(ss, msp)) vertex = 1;
+      else kind = 1;
+    } else if (tp_neg) {
+      if (dlt(tt, mtp)) vertex = 2;
+      else kind = 2;
+    }
+  } else if (region == 5) {
+    if (sp_neg) {
+      if (!dlt(msp, ss)) vertex = 1;
+      else kind = 1;
+    }
+  } else {
+    if (dlt(X, Y)) {  // s > t
+      if (dlt(den, num)) vertex = 2;
+      else kind = 4;
+    } else if (!gt0(Y)) {
+      vertex = 1;
+    } else if (sp_neg) {
+      kind = 1;
+    }
+  }
+  const double qn = kind == 5 ? 1.0 : (kind == 1 ? sp : (kind == 2 ? tp : (kind == 0 ? zero : num)));
+  const double qd = kind == 5 ? det : (kind == 1 ? ss : (kind == 2 ? tt : (kind == 0 ? 1.0 : den)));
+  const double q = qn / qd;
+  if (!in_range_of<600>(q)) return closest_dist_hw(tri, p);
+  const double q1 = 1.0 - q;
+  const double x = kind == 5 ? mul_int(s, q) : (kind == 1 || kind == 2 ? -q : (kind == 3 ? q : (kind == 4 ? q1 : zero)));
+  const double y = kind == 5 ? mul_int(t, q) : (kind == 3 ? q1 : (kind == 4 ? q : zero));
+  const bool ends = kind == 3 || kind == 4;
+  const d3 A = ends ? mk3(zero, zero, zero) : sel(kind == 0 && vertex == 1, v1, sel(kind == 0 && vertex == 2, v2, v0));
+  const d3 B = ends ? v1 : sel(kind == 2, tv, sv);
+  const d3 C = ends ? v2 : tv;
+  const d3 r = mk3((A.x + mul_int(x, B.x)) + mul_int(y, C.x), (A.y + mul_int(x, B.y)) + mul_int(y, C.y),
+                   (A.z + mul_int(x, B.z)) + mul_int(y, C.z));
+  const d3 w = sub3(r, p);
+  if (!(in_range_of<400>(w.x) && in_range_of<400>(w.y) && in_range_of<400>(w.z)))
+    return closest_dist_hw(tri, p);
+  return sqrt(dot_i(w, w));
+}
+
+// The mixed path makes 4.5 exact tests a point, mostly with few lanes of a
+// warp at once: the branches run less there and keep the kernel at 94
+// registers (five blocks an SM), which counts for more (1e6 points of the
+// nested spheres: 5.29 ms, 8.66 with closest_dist_i).  The all-FP64 path
+// tests every triangle it reaches, 78 a point: 18.3 -> 16.2 ms on 1e5 points,
+// and 11.5 with the box distances above (21.2 before both).
+template <bool MIXED>
+__device__ __forceinline__ double closest_dist(const double* tri, d3 p, bool safe) {
+  if (!MIXED) return safe ? closest_dist_i(tri, p) : closest_dist_hw(tri, p);
+  d3 v0, v1, v2;
+  load_tri64(tri, v0, v1, v2);
+  return dist64(closest64(v0, v1, v2, p), p);
+}
+
 // Whether (d, face) replaces (best, best_face): triangle_intersect.cpp:126-133
 // keeps a strictly nearer facet (strict <), and of facets at the same
 // distance the lowest face id wins.  (best, best_face) starts at (INFTY, -1),
@@ -263,7 +403,9 @@ __device__ __forceinline__ RecordBounds closest_record_bounds(const PlaneDists& 
 // order the candidates come in.
 __device__ __forceinline__ bool closest_better(double d, int32_t face, double best,
                                                int32_t best_face) {
-  return d < best || (d == best && best_face >= 0 && face < best_face);
+  // (distances are >= +0 or NaN: their bits order them, on the integer pipes)
+  const unsigned long long kd = (unsigned long long)dbits(d), kb = (unsigned long long)dbits(best);
+  return kd < kb || (kd == kb && best_face >= 0 && face < best_face);
 }
 
 // One lane per point, the warp in step: each round, every lane without a
@@ -295,6 +437,7 @@ __global__ void __launch_bounds__(kBlock) k_closest(PointArgs a) {
   d3 p = mk3(0.0, 0.0, 0.0);
   float px = 0.0f, py = 0.0f, pz = 0.0f, pabs = 0.0f, cmargin = 0.0f;
   bool f32ok = false, cbound = false;
+  bool safe = false;  // the point and the tree's vertices are in closest_dist_i's range
   int32_t ref = CHILD_EMPTY;
   bool run = false, deferred = false;
   int32_t steps = 0;  // node records and triangles of this point (a.step_budget)
@@ -314,6 +457,7 @@ __global__ void __launch_bounds__(kBlock) k_closest(PointArgs a) {
       // box test prunes nothing and every triangle gets the exact test
       f32ok = pabs + T.max_abs < 1e18f;
       cbound = MIXED && a.tri_cb && f32ok;
+      safe = !MIXED && T.int_ok != 0 && range60(p);
       cmargin = 48.0f * kU32 * (pabs + T.max_abs);
       ref = T.root;
       run = ref != CHILD_EMPTY;
@@ -339,19 +483,19 @@ __global__ void __launch_bounds__(kBlock) k_closest(PointArgs a) {
   float cl[kCand];
   int32_t cq[kCand];
   int nc = 0;
-  // the pruning bound: the best exact distance rounded up, or best_hi
-  auto bound = [&]() { return fminf(__double2float_ru(best), best_hi); };
+  // the pruning bound: bestf, the best exact distance rounded up, or best_hi
+  float bestf = INFINITY;
+  auto bound = [&]() { return fminf(bestf, best_hi); };
   // the exact closest-point test of leaf-ordered triangle qq
   auto exact = [&](int32_t qq) {
     if (MIXED) cnt.esc++;
-    d3 v0, v1, v2;
-    load_tri64(T.prim64 + kPrim64Stride * (int64_t)qq, v0, v1, v2);
-    const d3 r = closest64(v0, v1, v2, p);
-    const double dd = dist64(r, p);
+    const double* tri = T.prim64 + kPrim64Stride * (int64_t)qq;
+    const double dd = closest_dist<MIXED>(tri, p, safe);
     const int32_t fid = __ldg(&a.tri_face[__ldg(&T.prim_ref[qq])]);
     if (closest_better(dd, fid, best, best_face)) {
       best = dd;
       best_face = fid;
+      bestf = f32_up(best);
     }
   };
   // the next entry; one that can no longer hold a closer facet (its lower
@@ -391,8 +535,8 @@ __global__ void __launch_bounds__(kBlock) k_closest(PointArgs a) {
         ++steps;
         int32_t cr[4];
         float ck[4];
-        const int nhit = closest_children<MIXED>(T, ref, rec, p, px, py, pz, pabs, f32ok,
-                                                 fmin(best, (double)best_hi), cr, ck);
+        const int nhit = closest_children<MIXED>(T, ref, rec, p, px, py, pz, cmargin, f32ok,
+                                                 bound(), cr, ck);
         if (sp + nhit > kStackSize) {
           overflow = true;
           break;
@@ -541,8 +685,10 @@ __global__ void __launch_bounds__(32) k_closest_coop(PointArgs a) {
       const float pabs = fmaxf(fabsf(px), fmaxf(fabsf(py), fabsf(pz)));
       const bool f32ok = pabs + T.max_abs < 1e18f;
       const bool cbound = MIXED && a.tri_cb && f32ok;
+      const bool safe = !MIXED && T.int_ok != 0 && range60(p);
       const float cmargin = 48.0f * kU32 * (pabs + T.max_abs);
       double best = a.def_best[i];
+      float bestf = f32_up(best);
       int32_t best_face = a.def_face[i];
       int32_t st = RAY_OK;
       int top = 0;
@@ -559,7 +705,7 @@ __global__ void __launch_bounds__(32) k_closest_coop(PointArgs a) {
         // best (rounded up) holds no facet that could win
         const int take = min(top, 32);
         int32_t ref = CHILD_EMPTY;
-        if (lane < take && !(skey[top - 1 - lane] > __double2float_ru(best)))
+        if (lane < take && !(skey[top - 1 - lane] > bestf))
           ref = sref[top - 1 - lane];
         top -= take;
         __syncwarp();  // every entry read before the pushes below reuse the slots
@@ -575,8 +721,8 @@ __global__ void __launch_bounds__(32) k_closest_coop(PointArgs a) {
             cnt.box += 4;
             int32_t c4[4];
             float k4[4];
-            const int nh = closest_children<MIXED>(T, ref, rec, p, px, py, pz, pabs, f32ok, best,
-                                                   c4, k4);
+            const int nh = closest_children<MIXED>(T, ref, rec, p, px, py, pz, cmargin, f32ok,
+                                                   bestf, c4, k4);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               if (k < nh) {
@@ -590,7 +736,6 @@ __global__ void __launch_bounds__(32) k_closest_coop(PointArgs a) {
           }
         } else if (ref != CHILD_EMPTY) {
           const int32_t first = leaf_first(ref), count = leaf_count(ref);
-          const float bestf = __double2float_ru(best);
           for (int32_t q = 0; q < count; ++q) {
             cnt.prim++;
             const int32_t qq = first + q;
@@ -599,9 +744,8 @@ __global__ void __launch_bounds__(32) k_closest_coop(PointArgs a) {
                 continue;
               cnt.esc++;
             }
-            d3 v0, v1, v2;
-            load_tri64(T.prim64 + kPrim64Stride * (int64_t)qq, v0, v1, v2);
-            const double dd = dist64(closest64(v0, v1, v2, p), p);
+            const double* tri = T.prim64 + kPrim64Stride * (int64_t)qq;
+            const double dd = closest_dist<MIXED>(tri, p, safe);
             const int32_t fid = __ldg(&a.tri_face[__ldg(&T.prim_ref[qq])]);
             if (closest_better(dd, fid, lbest, lface)) {
               lbest = dd;
@@ -647,6 +791,7 @@ __global__ void __launch_bounds__(32) k_closest_coop(PointArgs a) {
           }
         }
         best = __shfl_sync(kFullMask, lbest, 0);
+        bestf = f32_up(best);
         best_face = __shfl_sync(kFullMask, lface, 0);
         if (st != RAY_OK) break;
       }

@@ -101,24 +101,6 @@ __device__ __forceinline__ void merge8(float* k, int32_t* r) {
 #undef XDG_CSWAP
 }
 
-__device__ __forceinline__ void sort4d(double* k, int32_t* r) {
-#define XDG_CSWAP(a, b)                 \
-  if (k[b] < k[a]) {                    \
-    double tk = k[a];                   \
-    k[a] = k[b];                        \
-    k[b] = tk;                          \
-    int32_t tr = r[a];                  \
-    r[a] = r[b];                        \
-    r[b] = tr;                          \
-  }
-  XDG_CSWAP(0, 1);
-  XDG_CSWAP(2, 3);
-  XDG_CSWAP(0, 2);
-  XDG_CSWAP(1, 3);
-  XDG_CSWAP(1, 2);
-#undef XDG_CSWAP
-}
-
 __device__ __forceinline__ float4 ld4(const float4* p) { return __ldg(p); }
 
 // FP32 ray data for the box test
