@@ -120,6 +120,27 @@ inline int device_sm_count() {
   return v;
 }
 
+// Items a warp takes (a power of two, 1 .. 32) in a launch of n items, so that
+// a batch too small to fill the lanes of `warps_per_sm` warps on every SM is
+// spread over about that many warps instead.  A warp takes as long as its
+// slowest item and steps through every branch its lanes take, so fewer items
+// a warp end sooner while the SMs have warps to spare: kSpreadWarps for
+// kernels that wait for memory.  The FP64 unit takes as long for one lane as
+// for 32, so launches that wait for it stop at kFp64Warps, about one and a
+// half warps a scheduler.  Measured with 32 items a warp and with the rule's:
+// mixed closest of 1,000 points 584 -> 202 us, 8,000 576 -> 354, 30,011 683 ->
+// 566 (65,000 at 16 instead of 32: 1071 against 832); mixed find_element of
+// 1,000 60 -> 31 us; mixed ray_fire of 1,000 rays of the nested spheres 122 ->
+// 92 us, 20,000 147 -> 136; all-FP64 ray_fire of 5,000 rays 225 -> 187 us
+// (20,000 at 8: 278 against 227); all-FP64 closest of 1,000 3.29 -> 2.14 ms.
+constexpr int kSpreadWarps = 16, kFp64Warps = 6;
+inline int lanes_per_warp(int64_t n, int warps_per_sm) {
+  const int64_t warps = (int64_t)device_sm_count() * warps_per_sm;
+  int lanes = 1;
+  while (lanes < 32 && lanes * warps < n) lanes *= 2;
+  return lanes;
+}
+
 // Resident blocks per SM of `kern` on the current device (`block` threads,
 // `smem` bytes of dynamic shared memory), looked up once per device in the
 // caller's `cache` (one per kernel variant and launch shape).

@@ -29,9 +29,12 @@ constexpr unsigned kFullMask = 0xffffffffu;
 // The point a thread of a point-query launch takes: its position in the
 // launch, or the entry of a.order there (a point index; an entry out of
 // range takes no point).
+// A warp takes a.lanes points, one per lane (the other lanes take none).
 __device__ __forceinline__ int64_t point_index(const PointArgs& a) {
-  const int64_t pos = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (!a.order || pos >= a.n) return pos;
+  const int64_t thread = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int lane = (int)(thread & 31);
+  const int64_t pos = lane < a.lanes ? (thread >> 5) * a.lanes + lane : a.n;
+  if (!a.order || pos >= a.n) return min(pos, a.n);
   const int32_t o = __ldg(&a.order[pos]);
   return o >= 0 ? (int64_t)o : a.n;
 }
@@ -1077,7 +1080,10 @@ __global__ void __launch_bounds__(kBlock) k_find_element(PointArgs a) {
   if (a.counters) flush_counters(a.counters, cnt, i < a.n ? 1ull : 0ull);
 }
 
-inline unsigned grid_for(int64_t n) { return (unsigned)((n + kBlock - 1) / kBlock); }
+inline unsigned grid_for(int64_t n, int lanes = 32) {
+  const int64_t warps = (n + lanes - 1) / lanes;
+  return (unsigned)((warps + kBlock / 32 - 1) / (kBlock / 32));
+}
 
 }  // namespace
 
@@ -1086,10 +1092,11 @@ cudaError_t launch_closest(bool mixed, const PointArgs& a, cudaStream_t st) {
   PointArgs b = a;
   const bool coop = a.step_budget > 0 && a.deferred && a.def_best && a.def_face;
   if (!coop) b.step_budget = 0;
+  b.lanes = lanes_per_warp(a.n, mixed ? kSpreadWarps : kFp64Warps);
   if (mixed)
-    k_closest<true><<<grid_for(a.n), kBlock, 0, st>>>(b);
+    k_closest<true><<<grid_for(a.n, b.lanes), kBlock, 0, st>>>(b);
   else
-    k_closest<false><<<grid_for(a.n), kBlock, 0, st>>>(b);
+    k_closest<false><<<grid_for(a.n, b.lanes), kBlock, 0, st>>>(b);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || !coop) return e;
   // the deferred points, one warp each; blocks of one warp with a 32 KB
@@ -1106,12 +1113,15 @@ cudaError_t launch_closest(bool mixed, const PointArgs& a, cudaStream_t st) {
 
 cudaError_t launch_find_element(bool mixed, const PointArgs& a, cudaStream_t st, bool phased) {
   if (a.n <= 0) return cudaSuccess;
+  PointArgs b = a;
+  b.lanes = lanes_per_warp(a.n, mixed && !phased ? kSpreadWarps : kFp64Warps);
+  const unsigned g = grid_for(a.n, b.lanes);
   if (mixed && phased)
-    k_find_element<true><<<grid_for(a.n), kBlock, 0, st>>>(a);
+    k_find_element<true><<<g, kBlock, 0, st>>>(b);
   else if (mixed)
-    k_find_element_lane<true><<<grid_for(a.n), kBlock, 0, st>>>(a);
+    k_find_element_lane<true><<<g, kBlock, 0, st>>>(b);
   else
-    k_find_element<false><<<grid_for(a.n), kBlock, 0, st>>>(a);
+    k_find_element<false><<<g, kBlock, 0, st>>>(b);
   return cudaGetLastError();
 }
 

@@ -112,6 +112,7 @@ struct PointArgs {
   // optional: position k of the launch takes point order[k] (a permutation
   // of 0..n-1; closest and find_element); results go to the point's own index
   const int32_t* order;
+  int32_t lanes;             // points a warp takes (1..32; set by the launch)
   double* dist_out;
   int32_t* id_out;
   int32_t* index_out;

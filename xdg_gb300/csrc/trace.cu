@@ -831,7 +831,12 @@ cudaError_t launch_minb(const SurfArgs& a, cudaStream_t st, int slot) {
         occupancy_cached(g_blocks_per_sm[slot][MINB - 2][a.stack / 8], kern, kTBlock, smem, per_sm);
     if (e != cudaSuccess) return e;
   }
-  const int64_t warps_needed = (a.n + 31) / 32;
+  // (a ray of these modes waits for memory; the rest wait for the FP64 unit,
+  // or restart in tree after tree, and do better with fuller warps)
+  constexpr bool spread = MIXED && (MODE == MODE_RAY_FIRE || MODE == MODE_PIV ||
+                                    MODE == MODE_OCCLUDED);
+  const int lanes = lanes_per_warp(a.n, spread ? kSpreadWarps : kFp64Warps);
+  const int64_t warps_needed = (a.n + lanes - 1) / lanes;
   int64_t blocks = (int64_t)device_sm_count() * per_sm;
   const int64_t max_blocks = (warps_needed + kTWarps - 1) / kTWarps;
   if (blocks > max_blocks) blocks = max_blocks;

@@ -1019,7 +1019,8 @@ cudaError_t launch_walk_s(const WalkArgs& a, cudaStream_t st) {
   const cudaError_t e = occupancy_cached(cached, kern, kBlock, 0, per_sm);
   if (e != cudaSuccess) return e;
   int64_t blocks = (int64_t)device_sm_count() * per_sm;
-  const int64_t max_blocks = (a.n + kBlock - 1) / kBlock;
+  const int lanes = a.order ? 32 : lanes_per_warp(a.n, kFp64Warps);
+  const int64_t max_blocks = ((a.n + lanes - 1) / lanes + kBlock / 32 - 1) / (kBlock / 32);
   if (blocks > max_blocks) blocks = max_blocks;
   if (blocks < 1) blocks = 1;
   const int64_t warps = blocks * (kBlock / 32);
@@ -1230,7 +1231,8 @@ cudaError_t launch_transport_t(const TransportArgs& a, cudaStream_t st) {
   const cudaError_t e = occupancy_cached(cached, kern, kBlock, 0, per_sm);
   if (e != cudaSuccess) return e;
   int64_t blocks = (int64_t)device_sm_count() * per_sm;
-  const int64_t max_blocks = (a.n + kBlock - 1) / kBlock;
+  const int lanes = lanes_per_warp(a.n, kFp64Warps);
+  const int64_t max_blocks = ((a.n + lanes - 1) / lanes + kBlock / 32 - 1) / (kBlock / 32);
   if (blocks > max_blocks) blocks = max_blocks;
   if (blocks < 1) blocks = 1;
   const int64_t warps = blocks * (kBlock / 32);
