@@ -446,13 +446,15 @@ int xdgcu_get_counters(xdgcu_ctx* ctx, int64_t counters[8]);
  *                      registers)
  *   "trace_node_iters" inner-node steps a lane takes between two leaf phases
  *                      of the warp-synchronous traversal, mixed precision
- *                      (1..64, default 4; the FP64 path's default is 1).  On
+ *                      (1..64, default 4; the FP64 path's default is 2).  On
  *                      the nested spheres every query ran fastest with 4 (1e7
  *                      rays, ms with 2/4/8/16 steps: ray_fire 7.36/6.50/
  *                      6.70/8.03, point_in_volume 7.05/6.23/6.41/7.71,
  *                      occluded 5.52/4.90/5.15/6.26, find_volume 22.6/22.1/
  *                      24.5/29.9)
- *   "trace_node_iters_fp64"  the same for the all-FP64 path
+ *   "trace_node_iters_fp64"  the same for the all-FP64 path (1e6 rays of the
+ *                      nested spheres, ms with 1/2/3/4/6 steps: 1.82/1.74/
+ *                      1.74/1.80/1.94)
  *   "trace_node_iters_direct"  the same for mixed calls whose rays the
  *                      kernel reads in place from host memory (host_direct;
  *                      default 6).  The best setting differs: 1e7 rays of
@@ -507,7 +509,7 @@ int xdgcu_get_counters(xdgcu_ctx* ctx, int64_t counters[8]);
  *                      sorted by length on the device and dealt round-robin
  *                      to warps, so warps end on short tracks.  Results do not
  *                      depend on it.
- *   "trace_edge_table" mixed ray_fire / point_in_volume / occluded /
+ *   "trace_edge_table" ray_fire / point_in_volume / occluded /
  *                      find_volume / particle loop: 1 (default) takes each
  *                      triangle's ray-independent FP64 terms (edge vectors,
  *                      edge normals, face normal) from a 256-byte record per
@@ -589,7 +591,7 @@ int xdgcu_get_counters(xdgcu_ctx* ctx, int64_t counters[8]);
  *                      that round's walks fit a buffer of about 1 GiB, so
  *                      rounds with fewer walks pause fewer of them).  Results
  *                      do not depend on it
- *   "walk_edge_table"  mixed walk: 1 (default) takes the FP64 Plucker
+ *   "walk_edge_table"  walk: 1 (default) takes the FP64 Plucker
  *                      coordinates of a face's edges from the edge table built
  *                      with the mesh (each edge's e and e x lo evaluated once,
  *                      the same values), 0 computes them from the vertices;

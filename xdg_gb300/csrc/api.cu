@@ -553,7 +553,7 @@ struct xdgcu_ctx {
   // tuning (xdgcu_set_tuning)
   int32_t trace_occupancy = 4;
   int32_t trace_node_iters = 4;       // mixed precision
-  int32_t trace_node_iters_fp64 = 1;  // all-FP64 path
+  int32_t trace_node_iters_fp64 = 2;  // all-FP64 path
   int32_t trace_node_iters_direct = 6;  // mixed launches reading their rays in place from host memory
   int32_t trace_flush_wait = 4;
   int32_t trace_stack = 40;      // shared-memory stack entries per lane
@@ -574,8 +574,8 @@ struct xdgcu_ctx {
   // all / the outputs of large calls' page-locked arrays, 5 (default) picks
   // 2, 3 or 4 for large calls by timing each (xdgcu_set_tuning)
   int32_t host_direct = 5;
-  int32_t walk_edge_table = 1;  // mixed walk: FP64 edge coordinates from the edge table
-  int32_t trace_edge_table = 1;  // mixed traversal: FP64 triangle terms from d_tri_prime
+  int32_t walk_edge_table = 1;  // walk: FP64 edge coordinates from the edge table
+  int32_t trace_edge_table = 1;  // traversal: FP64 triangle terms from d_tri_prime
   int32_t closest_bound = 1;     // mixed closest: FP32 triangle bound from d_tri_cb
   int32_t closest_node_steps = 4;       // closest: inner-node steps between leaf phases (mixed)
   int32_t closest_node_steps_fp64 = 1;  // the same, all-FP64 path

