@@ -559,6 +559,7 @@ struct xdgcu_ctx {
   int32_t trace_stack = 40;      // shared-memory stack entries per lane
   int32_t trace_grab = 0;        // 0: one contiguous chunk per warp; > 0: device work queue
   int64_t trace_sort_min = 0;    // batches of at least this many rays run in coherent order (0 = never)
+  int32_t surf_width8 = 0;            // some surface tree has 8-wide nodes
   int32_t surf_stack_bound = 0;       // largest (width - 1) * depth of the surface trees
   int32_t particle_event_wait = 16;  // particle_sim loop: lanes gathered before their events run
   int32_t transport_event_wait = 4;  // walk_elements tool loop (mixed): the same
@@ -673,8 +674,10 @@ int sync_tree_tables(xdgcu_ctx* c) {
   if (c->surf_trees_dirty) {
     std::vector<TreeDev> t;
     c->surf_stack_bound = 0;
+    c->surf_width8 = 0;
     for (auto& p : c->surf_trees) {
       t.push_back(p->dev);
+      if (p->dev.width == 8) c->surf_width8 = 1;
       // a traversal holds at most (width - 1) entries per inner level
       c->surf_stack_bound = std::max(c->surf_stack_bound, (p->dev.width - 1) * p->depth);
     }
@@ -2053,6 +2056,7 @@ static int surface_query(xdgcu_ctx* c, int mode, int32_t tree, const int32_t* ra
   a.surf_id = c->d_surf_id.p;
   a.surf_rev_tree = c->d_surf_rev.p;
   a.occupancy = c->trace_occupancy;
+  a.width8 = c->surf_width8;
   a.prim_edges = c->trace_edge_table;
   a.tri_prime = c->d_tri_prime.p;
   a.node_iters = precision == XDGCU_MIXED ? c->trace_node_iters : c->trace_node_iters_fp64;
@@ -2855,6 +2859,7 @@ int xdgcu_point_in_volumes(xdgcu_ctx* c, int64_t n, const double* points,
   a.surf_id = c->d_surf_id.p;
   a.surf_rev_tree = c->d_surf_rev.p;
   a.occupancy = c->trace_occupancy;
+  a.width8 = c->surf_width8;
   a.prim_edges = c->trace_edge_table;
   a.tri_prime = c->d_tri_prime.p;
   a.node_iters = precision == XDGCU_MIXED ? c->trace_node_iters : c->trace_node_iters_fp64;
@@ -2973,6 +2978,7 @@ int xdgcu_transport_surfaces(xdgcu_ctx* c, int64_t n, int32_t* tree, double* pos
   a.surf_bc = c->d_surf_bc.p;
   a.tri_xyz = c->d_tri_xyz.p;
   a.occupancy = c->trace_occupancy;
+  a.width8 = c->surf_width8;
   a.prim_edges = c->trace_edge_table;
   a.tri_prime = c->d_tri_prime.p;
   a.node_iters = precision == XDGCU_MIXED ? c->trace_node_iters : c->trace_node_iters_fp64;

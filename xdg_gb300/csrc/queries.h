@@ -47,6 +47,7 @@ struct SurfArgs {
   int32_t* status;
   unsigned long long* counters;
   int32_t occupancy;   // traversal kernel variant: minimum resident blocks per SM (2..4)
+  int32_t width8;      // some surface tree has 8-wide nodes
   int32_t node_iters;  // inner-node steps per lane between leaf phases (1..64)
   int32_t flush_wait;  // lanes waiting on the FP64 queue that force a partial drain (1..32)
   int32_t stack;       // shared-memory traversal stack entries per lane (16..64, multiple of 8)

@@ -76,8 +76,7 @@ struct WarpQueue {
   int32_t rsurf[32];
   int32_t rflags[32];  // bit 0: accepted, bit 1: dot(d, n) > 0
   int32_t rtri[32];    // global triangle of the result (particle mode: face normal)
-  uint32_t head, tail;
-  int32_t pad[2];
+  uint32_t mine[32];   // per lane: the drained entries whose owner it is
 };
 
 // Short-stack entries are node references, with (FP64 traversal only) the
@@ -138,7 +137,8 @@ __device__ __forceinline__ unsigned lanemask_lt() {
   return m;
 }
 
-template <int MODE, bool MIXED, int MINB>
+// W8: some surface tree may have 8-wide nodes (else all have 4-wide ones).
+template <int MODE, bool MIXED, int MINB, bool W8>
 __global__ void __launch_bounds__(kTBlock, MINB) k_trace(SurfArgs a, int64_t chunk) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31;
@@ -178,10 +178,8 @@ __global__ void __launch_bounds__(kTBlock, MINB) k_trace(SurfArgs a, int64_t chu
   int64_t cursor = dyn ? 0 : gwarp * chunk;
   int64_t end = dyn ? 0 : min(a.n, cursor + chunk);
   bool exhausted = false;  // work queue (grab > 0) has no rays left
-  if (lane == 0) {
-    Q.head = 0u;
-    Q.tail = 0u;
-  }
+  uint32_t qhead = 0u, qtail = 0u;  // of the warp's queue (warp-uniform)
+  Q.mine[lane] = 0u;
   __syncwarp();
 
   Counters cnt = {0, 0, 0, 0};
@@ -266,7 +264,7 @@ __global__ void __launch_bounds__(kTBlock, MINB) k_trace(SurfArgs a, int64_t chu
     tree = T;
     n32 = T->n32;
     prim32 = T->prim32;
-    wide8 = T->width == 8;
+    wide8 = W8 && T->width == 8;
     const int32_t root = T->root;
     bt32 = (MODE == MODE_OCCLUDED) ? INFINITY : f32_up(bt);
     if (MIXED) {
@@ -284,6 +282,17 @@ __global__ void __launch_bounds__(kTBlock, MINB) k_trace(SurfArgs a, int64_t chu
       leaf_end = leaf_p + leaf_count(root);
     } else {
       cur = root;
+    }
+  };
+
+  // near distances (FP32, +inf for misses) and references of the children of
+  // 4-wide record `rec` of the lane's tree
+  auto node_test = [&](int64_t rec, float* key, int32_t* ref) {
+    if (MIXED && !use64) {
+      node_test32(n32 + rec, br32, bt32, key, ref);
+    } else {
+      if (MIXED) br64 = make_boxray64(ray_o(tx), ray_d(tx));  // rare: rays failing the FP32 safety test
+      node_test64(tree->n64 + rec, br64, (MODE == MODE_OCCLUDED) ? INFTY : bt, key, ref);
     }
   };
 
@@ -561,34 +570,64 @@ __global__ void __launch_bounds__(kTBlock, MINB) k_trace(SurfArgs a, int64_t chu
       if (want) {
         cnt.node++;
         cnt.box += wide8 ? 8 : 4;
-        // an 8-wide node is two 4-wide records, each tested and sorted, then
-        // merged; a 4-wide node leaves the upper half empty
-        int32_t cr[8];
-        float key[8];
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          if (r == 1 && !wide8) {
-#pragma unroll
-            for (int k = 4; k < 8; ++k) {
-              key[k] = INFINITY;
-              cr[k] = CHILD_EMPTY;
-            }
-            continue;
-          }
-          const int64_t rec = wide8 ? 2 * (int64_t)cur + r : (int64_t)cur;
-          if (MIXED && !use64) {
-            node_test32(n32 + rec, br32, bt32, key + 4 * r, cr + 4 * r);
-          } else {
-            if (MIXED) br64 = make_boxray64(ray_o(tx), ray_d(tx));  // rare: rays failing the FP32 safety test
-            node_test64(tree->n64 + rec, br64, (MODE == MODE_OCCLUDED) ? INFTY : bt, key + 4 * r,
-                        cr + 4 * r);
-          }
-          sort4(key + 4 * r, cr + 4 * r);
-        }
-        if (wide8) merge8(key, cr);
+        // the children hit, nearest first: nhit of them, their references in
+        // cr and the upper 16 bits of their near distances in kb
+        int32_t cr[W8 ? 8 : 4];
+        uint32_t kb[W8 ? 8 : 4];
         int nhit = 0;
+        if (W8) {
+          // an 8-wide node is two 4-wide records, each tested and sorted, then
+          // merged; a 4-wide node leaves the upper half empty
+          float key[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) nhit += key[k] < INFINITY ? 1 : 0;
+          for (int r = 0; r < 2; ++r) {
+            if (r == 1 && !wide8) {
+#pragma unroll
+              for (int k = 4; k < 8; ++k) {
+                key[k] = INFINITY;
+                cr[W8 ? k : 0] = CHILD_EMPTY;
+              }
+              continue;
+            }
+            const int64_t rec = wide8 ? 2 * (int64_t)cur + r : (int64_t)cur;
+            node_test(rec, key + 4 * r, cr + 4 * (W8 ? r : 0));
+            sort4(key + 4 * r, cr + 4 * (W8 ? r : 0));
+          }
+          if (wide8) merge8(key, cr);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            nhit += key[k] < INFINITY ? 1 : 0;
+            kb[W8 ? k : 0] = __float_as_uint(key[k]) >> 16;
+          }
+        } else {
+          // the four near distances (>= 0, +inf: a miss) sorted as integers
+          // with the child's slot in the two lowest bits
+          float key[4];
+          int32_t ref[4];
+          node_test(cur, key, ref);
+          constexpr uint32_t kMiss = 0x7f800000u;
+          uint32_t p[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) p[k] = (__float_as_uint(key[k]) & 0x7ffffffcu) | (uint32_t)k;
+          auto order = [&](int x, int y) {
+            const uint32_t lo = min(p[x], p[y]);
+            p[y] = max(p[x], p[y]);
+            p[x] = lo;
+          };
+          order(0, 1);
+          order(2, 3);
+          order(0, 2);
+          order(1, 3);
+          order(1, 2);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            nhit += p[k] < kMiss ? 1 : 0;
+            const uint32_t slot = p[k] & 3u;
+            const int32_t lo = (slot & 1u) ? ref[1] : ref[0], hi = (slot & 1u) ? ref[3] : ref[2];
+            cr[k] = (slot & 2u) ? hi : lo;
+            kb[k] = p[k] >> 16;
+          }
+        }
         if (nhit == 0) {
           pop();
         } else if (sp + nhit - 1 > kstack) {
@@ -596,10 +635,10 @@ __global__ void __launch_bounds__(kTBlock, MINB) k_trace(SurfArgs a, int64_t chu
           trav = false;
         } else {
 #pragma unroll
-          for (int k = 7; k >= 1; --k) {
-            if (k < nhit) {  // static indices keep key/cr in registers
+          for (int k = (W8 ? 7 : 3); k >= 1; --k) {
+            if (k < nhit) {  // static indices keep cr in registers
               sref[sp * kTBlock + tx] = cr[k];
-              if (kKeys) stn[sp * kTBlock + tx] = (uint16_t)(__float_as_uint(key[k]) >> 16);
+              if (kKeys) stn[sp * kTBlock + tx] = (uint16_t)kb[k];
               ++sp;
             }
           }
@@ -638,20 +677,15 @@ __global__ void __launch_bounds__(kTBlock, MINB) k_trace(SurfArgs a, int64_t chu
       }
       if (cur == CHILD_EMPTY) pop();
     }
-    // ---- enqueue this step's escalations (warp-wide exclusive scan) ----
+    // ---- enqueue this step's escalations (at most 4 a lane: their prefix
+    // sums from the ballots of the count's three bits) ----
     {
       const int c = __popc(escm);
-      int incl = c;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const int y = __shfl_up_sync(kFull, incl, off);
-        if (lane >= off) incl += y;
-      }
-      const int total = __shfl_sync(kFull, incl, 31);
-      if (total > 0) {
-        const uint32_t tail = Q.tail;
-        __syncwarp();
-        uint32_t pos = tail + (uint32_t)(incl - c);
+      const unsigned b0 = __ballot_sync(kFull, c & 1), b1 = __ballot_sync(kFull, c & 2),
+                     b2 = __ballot_sync(kFull, c & 4);
+      if ((b0 | b1 | b2) != 0u) {
+        const unsigned lt = lanemask_lt();
+        uint32_t pos = qtail + (uint32_t)(__popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt));
         unsigned m = escm;
         while (m) {
           const int k = __ffs(m) - 1;
@@ -661,15 +695,15 @@ __global__ void __launch_bounds__(kTBlock, MINB) k_trace(SurfArgs a, int64_t chu
         }
         npend += c;
         cnt.esc += c;
-        if (lane == 0) Q.tail = tail + (uint32_t)total;
+        qtail += (uint32_t)(__popc(b0) + 2 * __popc(b1) + 4 * __popc(b2));
       }
     }
     __syncwarp();
 
     // ---- drain the FP64 queue with the whole warp ----
     while (true) {
-      const uint32_t head = Q.head;
-      const int qn = (int)(Q.tail - head);
+      const uint32_t head = qhead;
+      const int qn = (int)(qtail - head);
       const unsigned act2 = __ballot_sync(kFull, trav);
       const unsigned waiting = __ballot_sync(kFull, has_ray && !trav && npend > 0);
       if (!(qn >= 32 || (qn > 0 && (act2 == 0u || __popc(waiting) >= a.flush_wait)))) break;
@@ -762,13 +796,15 @@ __global__ void __launch_bounds__(kTBlock, MINB) k_trace(SurfArgs a, int64_t chu
       Q.rface[lane] = rface;
       Q.rsurf[lane] = rsurf;
       if (MODE == MODE_PARTICLE) Q.rtri[lane] = rtri;
-      const int my_owner = owner;
+      if (mine) atomicOr(&Q.mine[owner], 1u << lane);
       __syncwarp();
-      // each ray merges its own results in queue order
+      // each ray merges its own results, in queue order
       bool changed = false;
-      for (int j = 0; j < nq; ++j) {
-        if (__shfl_sync(kFull, my_owner, j) != lane) continue;
-        npend--;
+      unsigned own = Q.mine[lane];
+      Q.mine[lane] = 0u;
+      npend -= __popc(own);
+      for (; own != 0u; own &= own - 1u) {
+        const int j = __ffs(own) - 1;
         const int32_t fl = Q.rflags[j];
         if (!(fl & 1)) continue;
         if (MODE == MODE_OCCLUDED) {
@@ -790,8 +826,7 @@ __global__ void __launch_bounds__(kTBlock, MINB) k_trace(SurfArgs a, int64_t chu
         }
       }
       if (changed) bt32 = f32_up(bt);
-      __syncwarp();
-      if (lane == 0) Q.head = head + (uint32_t)nq;
+      qhead = head + (uint32_t)nq;
       __syncwarp();
     }
   }
@@ -804,29 +839,31 @@ __global__ void __launch_bounds__(kTBlock, MINB) k_trace(SurfArgs a, int64_t chu
 // resident blocks per SM, by kernel variant, MINB and stack depth (8..64
 // step 8), per device, and whether the variant's shared-memory limit is
 // raised on a device; filled on first use, from any host thread
-std::atomic<int> g_blocks_per_sm[12][3][kTStackMax / 8 + 1][kMaxDevices];
-std::atomic<bool> g_smem_attr[12][3][kMaxDevices];
+// (variants 2..4 blocks per SM for trees of either width, then 4 for 4-wide ones)
+std::atomic<int> g_blocks_per_sm[12][4][kTStackMax / 8 + 1][kMaxDevices];
+std::atomic<bool> g_smem_attr[12][4][kMaxDevices];
 
-template <int MODE, bool MIXED, int MINB>
+template <int MODE, bool MIXED, int MINB, bool W8>
 cudaError_t launch_minb(const SurfArgs& a, cudaStream_t st, int slot) {
+  constexpr int kVar = W8 ? MINB - 2 : 3;
   if (a.stack < kTStackMin || a.stack > kTStackMax || a.stack % 8 != 0) return cudaErrorInvalidValue;
   if (a.grab > 0 && (a.work == nullptr || a.grab % 32 != 0)) return cudaErrorInvalidValue;
   constexpr bool keys = stack_keys<MODE, MIXED>();
   const size_t smem = trace_smem_bytes(a.stack, keys, MODE == MODE_PARTICLE && MIXED);
-  auto kern = k_trace<MODE, MIXED, MINB>;
+  auto kern = k_trace<MODE, MIXED, MINB, W8>;
   const int dev = current_device();
   const bool known = dev >= 0 && dev < kMaxDevices;
-  if (!known || !g_smem_attr[slot][MINB - 2][dev].load(std::memory_order_acquire)) {
+  if (!known || !g_smem_attr[slot][kVar][dev].load(std::memory_order_acquire)) {
     cudaError_t e = cudaFuncSetAttribute(
         kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
         (int)trace_smem_bytes(kTStackMax, keys, MODE == MODE_PARTICLE && MIXED));
     if (e != cudaSuccess) return e;
-    if (known) g_smem_attr[slot][MINB - 2][dev].store(true, std::memory_order_release);
+    if (known) g_smem_attr[slot][kVar][dev].store(true, std::memory_order_release);
   }
   int per_sm = 0;
   {
     const cudaError_t e =
-        occupancy_cached(g_blocks_per_sm[slot][MINB - 2][a.stack / 8], kern, kTBlock, smem, per_sm);
+        occupancy_cached(g_blocks_per_sm[slot][kVar][a.stack / 8], kern, kTBlock, smem, per_sm);
     if (e != cudaSuccess) return e;
   }
   // (a ray of these modes waits for memory; the rest wait for the FP64 unit,
@@ -848,9 +885,14 @@ cudaError_t launch_minb(const SurfArgs& a, cudaStream_t st, int slot) {
 template <int MODE, bool MIXED>
 cudaError_t launch_one(const SurfArgs& a, cudaStream_t st, int slot) {
   switch (a.occupancy) {
-    case 2: return launch_minb<MODE, MIXED, 2>(a, st, slot);
-    case 4: return launch_minb<MODE, MIXED, 4>(a, st, slot);
-    default: return launch_minb<MODE, MIXED, 3>(a, st, slot);
+    case 2: return launch_minb<MODE, MIXED, 2, true>(a, st, slot);
+    case 4:
+      // the code for 8-wide nodes costs a third of a 4-wide node step's
+      // instructions, so 4-wide trees have their own kernel at the default
+      // occupancy
+      return a.width8 ? launch_minb<MODE, MIXED, 4, true>(a, st, slot)
+                      : launch_minb<MODE, MIXED, 4, false>(a, st, slot);
+    default: return launch_minb<MODE, MIXED, 3, true>(a, st, slot);
   }
 }
 
