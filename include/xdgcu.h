@@ -471,17 +471,24 @@ int xdgcu_get_counters(xdgcu_ctx* ctx, int64_t counters[8]);
  *                      which no traversal can exceed, up to 64; only trees
  *                      deeper than that can make a ray end with
  *                      XDGCU_RAY_STACK_OVERFLOW
- *   "trace_grab"       0 (default): each warp walks one contiguous slice of
- *                      the batch fixed at launch; > 0 (a multiple of 32): warps
- *                      take this many rays at a time from a device work queue,
- *                      which balances batches of very uneven per-ray cost
+ *   "trace_grab"       > 0 (a multiple of 32): warps take this many rays at a
+ *                      time from a device work queue, which balances batches of
+ *                      very uneven per-ray cost; 0 (default): by the batch --
+ *                      mixed ray_fire, point_in_volume and occluded of at least
+ *                      2e6 rays take 64 at a time, find_volume and
+ *                      point_in_volumes of at least 5e5 points 32, and other
+ *                      launches (and those captured in a graph) give each warp
+ *                      one contiguous slice fixed at launch
  *   "particle_event_wait"  particle loop of xdgcu_transport_surfaces: lanes
  *                      whose flights have ended that a warp gathers before it
- *                      runs their events together (1..32, default 16)
- *   "transport_event_wait" particle loop of xdgcu_transport_elements, mixed
- *                      precision: lanes whose events need the FP64 sample
- *                      (collisions, uncertain exits) that a warp gathers
- *                      before it runs them together (1..32, default 4)
+ *                      runs their events together (1..32, default 20: 1e6
+ *                      particles of the nested spheres 76.4 / 76.2 / 78.9 ms
+ *                      with 16 / 20 / 24)
+ *   "transport_event_wait" particle loop of xdgcu_transport_elements: lanes
+ *                      whose events need the FP64 sample (collisions,
+ *                      uncertain exits) that a warp gathers before it runs
+ *                      them together, in batches that give every lane a
+ *                      particle (1..32, default 4; smaller batches never wait)
  *   "trace_sort_min"   batches of at least this many rays (default 0 = never)
  *                      are traversed in a coherent order: sorted on the device
  *                      by tree, direction octant and the Morton code of the

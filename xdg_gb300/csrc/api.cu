@@ -561,7 +561,7 @@ struct xdgcu_ctx {
   int64_t trace_sort_min = 0;    // batches of at least this many rays run in coherent order (0 = never)
   int32_t surf_width8 = 0;            // some surface tree has 8-wide nodes
   int32_t surf_stack_bound = 0;       // largest (width - 1) * depth of the surface trees
-  int32_t particle_event_wait = 16;  // particle_sim loop: lanes gathered before their events run
+  int32_t particle_event_wait = 20;  // particle_sim loop: lanes gathered before their events run
   int32_t transport_event_wait = 4;  // walk_elements tool loop (mixed): the same
   int32_t leaf_max = 2;
   int32_t node_width = 4;        // children per BVH node (4 or 8) of trees built afterwards
@@ -1396,12 +1396,33 @@ int32_t trace_stack_for(const xdgcu_ctx* c) {
   return std::max(c->trace_stack, need);
 }
 
+// Rays a warp takes at a time from the device work queue where trace_grab
+// leaves the choice open (0), or 0 for fixed slices.  The queue evens out the
+// ends of large batches; its counter has to be allocated and zeroed, and with
+// few rays a warp the last chunks are uneven work again.  Nested spheres, ms
+// with slices / 32 / 64 rays: ray_fire of 1e6 0.686 / 0.677 / 0.689, 2e6 1.265 /
+// 1.220 / 1.229, 1e7 5.685 / 5.543 / 5.487; point_in_volume of 4e6 2.372 / 2.283 /
+// 2.272; find_volume of 2e5 0.793 / 0.821 / 0.920, 5e5 1.419 / 1.378 / 1.472, 5e6
+// 10.23 / 9.58 / 9.62.  A captured launch keeps the slices (its counter would
+// be the graph's).
+int32_t queue_grab_for(int mode, bool mixed, int64_t n, cudaStream_t s) {
+  const bool restarts = mode == MODE_FIND_VOLUME || mode == MODE_ALL_VOLUMES;
+  if (!mixed || mode == MODE_PARTICLE || n < (restarts ? 500000 : 2000000)) return 0;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return cap != cudaStreamCaptureStatusNone ? 0 : (restarts ? 32 : 64);
+}
+
 cudaError_t launch_trace(xdgcu_ctx* c, int mode, bool mixed, SurfArgs a, double extent,
                          cudaStream_t s, int32_t min_grab = 0) {
   if (a.n <= 0) return cudaSuccess;
   const bool sort = c->trace_sort_min > 0 && a.n >= c->trace_sort_min && a.n < ((int64_t)1 << 31) &&
                     extent > 0.0;
   a.grab = std::max(c->trace_grab, min_grab);
+  if (a.grab == 0) a.grab = queue_grab_for(mode, mixed, a.n, s);
   a.work = nullptr;
   a.order = nullptr;
   if (a.grab == 0 && !sort) return launch_surface_query(mode, mixed, a, s);
@@ -2990,6 +3011,10 @@ int xdgcu_transport_surfaces(xdgcu_ctx* c, int64_t n, int32_t* tree, double* pos
   a.hist_cap = history_cap;
   a.event_wait = c->particle_event_wait;
   const bool mixed = precision == XDGCU_MIXED;
+  // Where every lane has a particle, the others' work covers a longer wait for
+  // fuller drains (1e6 particles of the nested spheres, event_wait 20: 79.9 ms
+  // flushing at 4 waiting lanes, 76.2 at 8; 20,000 particles 17.1 and 17.4)
+  if (mixed && n >= (int64_t)device_sm_count() * 16 * 32) a.flush_wait = std::max(a.flush_wait, 8);
   cudaStream_t st = (cudaStream_t)stream;
   auto bind = [&](char* const* p) {
     a.p_tree = (int32_t*)p[0];
@@ -3086,9 +3111,11 @@ int xdgcu_transport_elements(xdgcu_ctx* c, int64_t n, int32_t* elem_index, doubl
   t.n = n;
   t.mfp = mean_free_path;
   t.max_events = max_events;
-  // FP64 steps are FP64-bound themselves: idle waiting lanes cost more than
-  // the batching saves, so the all-FP64 loop runs each event at once
-  t.event_wait = precision == XDGCU_MIXED ? c->transport_event_wait : 1;
+  // Waiting for fuller batches of collisions pays once every lane has a
+  // particle; before that the lanes that wait are what the launch waits for
+  // (ms with 1 / 2 / 4 lanes, mixed: 20,000 particles 11.5 / 12.1 / 12.2, 200,000
+  // 25.7 / 23.8 / 23.6; FP64: 14.8 / 15.6 / 15.8 and 34.0 / 32.2 / 32.6)
+  t.event_wait = n >= (int64_t)device_sm_count() * 16 * 32 ? c->transport_event_wait : 1;
   const bool mixed = precision == XDGCU_MIXED;
   cudaStream_t st = (cudaStream_t)stream;
   if (kind == 1) {
