@@ -411,7 +411,7 @@ __global__ void k_tet_boxes(const double* __restrict__ xyz, const int4* __restri
   }
 }
 
-// Leaf-ordered tet data.  prim64: the 4 vertices (12 doubles).  prim32: the
+// Leaf-ordered tet data.  prim64: tet_inverse64's 12 doubles.  prim32: the
 // data of the FP32 containment pre-filter (geom.cuh, tet_filter32):
 //   float4 (v0.xyz, m)  (M row 0, |v0|_inf)  (M row 1, e64)  (M row 2, 0)
 // with M = T^{-1} (T's columns v1-v0, v2-v0, v3-v0) rounded to FP32,
@@ -428,12 +428,11 @@ __global__ void k_tet_gather(const double* __restrict__ xyz, const int4* __restr
   const int4 c = conn[t];
   const int32_t ci[4] = {c.x, c.y, c.z, c.w};
   double v[4][3];
-  double* o = prim64 + 12 * (int64_t)j;
   for (int k = 0; k < 4; ++k)
-    for (int a = 0; a < 3; ++a) {
-      v[k][a] = xyz[3 * (int64_t)ci[k] + a];
-      o[3 * k + a] = v[k][a];
-    }
+    for (int a = 0; a < 3; ++a) v[k][a] = xyz[3 * (int64_t)ci[k] + a];
+  tet_inverse64(mk3(v[0][0], v[0][1], v[0][2]), mk3(v[1][0], v[1][1], v[1][2]),
+                mk3(v[2][0], v[2][1], v[2][2]), mk3(v[3][0], v[3][1], v[3][2]),
+                prim64 + 12 * (int64_t)j);
   prim_ref[j] = t;
   // T[r][col]: column col = v_{col+1} - v0
   double T[3][3], Tmax = 0.0, lo[3], hi[3];
@@ -580,7 +579,7 @@ struct xdgcu_ctx {
   int32_t closest_bound = 1;     // mixed closest: FP32 triangle bound from d_tri_cb
   int32_t closest_node_steps = 4;       // closest: inner-node steps between leaf phases (mixed)
   int32_t closest_node_steps_fp64 = 1;  // the same, all-FP64 path
-  int32_t find_node_steps_fp64 = 16;    // find_element in phases (all-FP64, or find_phased): the same
+  int32_t find_node_steps_fp64 = 4;    // find_element in phases (all-FP64, or find_phased): the same
   int32_t find_phased = 0;  // mixed find_element: 1 runs warp-synchronous phases, 0 one lane per point
   int32_t packed_passes = 1;  // packed walk: 1 walk in resumed rounds, 2 a count walk and an emit walk
   int32_t closest_budget = 1024;  // closest: steps of one lane before a warp takes the point (0: never)

@@ -239,18 +239,36 @@ __device__ __forceinline__ int normal_dot_sign(d3 d, d3 v0, d3 v1, d3 v2) {
 // tetrahedron_contain.cpp:11-43.  The reference solves T*lambda = p - v0 with
 // T's columns e0 = v1-v0, e1 = v2-v0, e2 = v3-v0 through its linalg
 // dependency: inverse = adjugate / determinant, then mul(inverse, rhs) summed
-// over columns.  The same formula and order are used here.
-__device__ __forceinline__ bool tet_contains64(d3 p, d3 v0, d3 v1, d3 v2, d3 v3) {
+// over columns.  The same formula and order are used here.  The inverse does
+// not depend on the point: tet_inverse64 evaluates it once per tet when its
+// tree is built (12 doubles: v0 and the inverse's three columns, in place of
+// the four vertices), and the test takes 21 FP64 operations instead of about
+// 150, nine divisions among them.
+__device__ __forceinline__ void tet_inverse64(d3 v0, d3 v1, d3 v2, d3 v3, double* out) {
   const d3 X = sub3(v1, v0), Y = sub3(v2, v0), Z = sub3(v3, v0);
   const d3 ax = mk3(Y.y * Z.z - Z.y * Y.z, Z.y * X.z - X.y * Z.z, X.y * Y.z - Y.y * X.z);
   const d3 ay = mk3(Y.z * Z.x - Z.z * Y.x, Z.z * X.x - X.z * Z.x, X.z * Y.x - Y.z * X.x);
   const d3 az = mk3(Y.x * Z.y - Z.x * Y.y, Z.x * X.y - X.x * Z.y, X.x * Y.y - Y.x * X.y);
   const double det = X.x * (Y.y * Z.z - Z.y * Y.z) + X.y * (Y.z * Z.x - Z.z * Y.x) +
                      X.z * (Y.x * Z.y - Z.x * Y.y);
-  const d3 ix = mk3(ax.x / det, ax.y / det, ax.z / det);
-  const d3 iy = mk3(ay.x / det, ay.y / det, ay.z / det);
-  const d3 iz = mk3(az.x / det, az.y / det, az.z / det);
-  const d3 rhs = sub3(p, v0);
+  out[0] = v0.x;
+  out[1] = v0.y;
+  out[2] = v0.z;
+  const d3 col[3] = {ax, ay, az};
+  for (int k = 0; k < 3; ++k) {
+    out[3 + 3 * k] = col[k].x / det;
+    out[4 + 3 * k] = col[k].y / det;
+    out[5 + 3 * k] = col[k].z / det;
+  }
+}
+
+// R: tet_inverse64's 12 doubles
+__device__ __forceinline__ bool tet_contains64(d3 p, const double* R) {
+  const double2* q = reinterpret_cast<const double2*>(R);
+  const double2 r0 = __ldg(q), r1 = __ldg(q + 1), r2 = __ldg(q + 2), r3 = __ldg(q + 3),
+                r4 = __ldg(q + 4), r5 = __ldg(q + 5);
+  const d3 ix = mk3(r1.y, r2.x, r2.y), iy = mk3(r3.x, r3.y, r4.x), iz = mk3(r4.y, r5.x, r5.y);
+  const d3 rhs = sub3(p, mk3(r0.x, r0.y, r1.x));
   const d3 l = add3(add3(scl3(rhs.x, ix), scl3(rhs.y, iy)), scl3(rhs.z, iz));
   const double l0 = 1.0 - (l.x + l.y + l.z);
   // bary < -PLUCKER_ZERO_TOL || bary > 1.0f + PLUCKER_ZERO_TOL, on integer keys

@@ -60,7 +60,7 @@ enum TreeKind : int32_t { TREE_SURFACE = 0, TREE_ELEMENT = 1 };
 //                     (v2-v0, 1 if well shaped at v0 for closest's upper bound, else 0)
 //                  prim64 = 10 doubles per triangle (v0, v1, v2, pad)
 //                  prim_ref = global triangle index
-//   element trees: prim64 = 12 doubles per tet (v0..v3), prim_ref = tet index
+//   element trees: prim64 = 12 doubles per tet (tet_inverse64), prim_ref = tet index
 // Surface trees also hold, per 4-wide record, 16 float4 for closest (cobb.h):
 // the child references, then for each of three axes the four children's row
 // x, y, z, middle d and half width h.

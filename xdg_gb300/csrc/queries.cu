@@ -813,6 +813,13 @@ __global__ void __launch_bounds__(32) k_closest_coop(PointArgs a) {
 // find_element (embree/ray_tracer.cpp:226-257 + tetrahedron_contain.cpp:94-114)
 // ---------------------------------------------------------------------------
 
+// whether p is in child k's FP64 box, compared on the integer pipes
+__device__ __forceinline__ bool in_box64(const Node64* np, int k, d3 p) {
+  return !dlt(p.x, __ldg(np->lox + k)) && !dlt(__ldg(np->hix + k), p.x) &&
+         !dlt(p.y, __ldg(np->loy + k)) && !dlt(__ldg(np->hiy + k), p.y) &&
+         !dlt(p.z, __ldg(np->loz + k)) && !dlt(__ldg(np->hiz + k), p.z);
+}
+
 // One thread per point, each on its own: the mixed path, whose FP32 filter
 // decides nearly every tet of an interior point, runs faster this way (1409
 // against 1249 Mpoints/s in warp-synchronous phases, 1e6 uniform points in
@@ -867,12 +874,8 @@ __global__ void __launch_bounds__(kBlock) k_find_element_lane(PointArgs a) {
             const Node64* np = T.n64 + (int64_t)ref * nrec + rec;
             const int4 c = __ldg(&np->child);
             const int32_t ca[4] = {c.x, c.y, c.z, c.w};
-            for (int k = 0; k < 4; ++k) {
-              const bool in = p.x >= __ldg(np->lox + k) && p.x <= __ldg(np->hix + k) &&
-                              p.y >= __ldg(np->loy + k) && p.y <= __ldg(np->hiy + k) &&
-                              p.z >= __ldg(np->loz + k) && p.z <= __ldg(np->hiz + k);
-              if (in) cr[nhit++] = ca[k];
-            }
+            for (int k = 0; k < 4; ++k)
+              if (in_box64(np, k, p)) cr[nhit++] = ca[k];
           }
           if (sp + nhit > kStackSize) {
             overflow = true;
@@ -904,12 +907,7 @@ __global__ void __launch_bounds__(kBlock) k_find_element_lane(PointArgs a) {
               }
               cnt.esc++;
             }
-            const double* v = T.prim64 + 12 * (int64_t)q;
-            const d3 v0 = mk3(__ldg(v + 0), __ldg(v + 1), __ldg(v + 2));
-            const d3 v1 = mk3(__ldg(v + 3), __ldg(v + 4), __ldg(v + 5));
-            const d3 v2 = mk3(__ldg(v + 6), __ldg(v + 7), __ldg(v + 8));
-            const d3 v3 = mk3(__ldg(v + 9), __ldg(v + 10), __ldg(v + 11));
-            if (!tet_contains64(p, v0, v1, v2, v3)) continue;
+            if (!tet_contains64(p, T.prim64 + 12 * (int64_t)q)) continue;
             const int32_t idx = __ldg(&T.prim_ref[q]);
             const int32_t id = __ldg(&a.elem_ids[idx]);
             if (best_idx < 0 || id < best_id) {  // tie rule: lowest element id
@@ -935,8 +933,10 @@ __global__ void __launch_bounds__(kBlock) k_find_element_lane(PointArgs a) {
 // containment tests of all the warp's lanes together.  Every containing tet
 // is visited (the lowest element id wins), so no entry is pruned.  The
 // all-FP64 path, where every tet of a leaf takes the exact test, runs this
-// way: 76.5 -> 114 Mpoints/s with 16 node steps (1e6 points, 750,000 tets);
-// so does the mixed path for points on tet faces (launch_find_element).
+// way, and so does the mixed path for points on tet faces
+// (launch_find_element).  With the tets' inverses stored and the boxes compared
+// on the integer pipes the all-FP64 path takes 2.39 ms for 2e6 points of the
+// 750,000-tet cube, where it took 16.5 from the vertices.
 template <bool MIXED>
 __global__ void __launch_bounds__(kBlock) k_find_element(PointArgs a) {
   const int64_t i = point_index(a);
@@ -1013,12 +1013,8 @@ __global__ void __launch_bounds__(kBlock) k_find_element(PointArgs a) {
           const Node64* np = T.n64 + (int64_t)ref * nrec + rec;
           const int4 c = __ldg(&np->child);
           const int32_t ca[4] = {c.x, c.y, c.z, c.w};
-          for (int k = 0; k < 4; ++k) {
-            const bool in = p.x >= __ldg(np->lox + k) && p.x <= __ldg(np->hix + k) &&
-                            p.y >= __ldg(np->loy + k) && p.y <= __ldg(np->hiy + k) &&
-                            p.z >= __ldg(np->loz + k) && p.z <= __ldg(np->hiz + k);
-            if (in) cr[nhit++] = ca[k];
-          }
+          for (int k = 0; k < 4; ++k)
+            if (in_box64(np, k, p)) cr[nhit++] = ca[k];
         }
         if (sp + nhit > kStackSize) {
           overflow = true;
@@ -1062,12 +1058,7 @@ __global__ void __launch_bounds__(kBlock) k_find_element(PointArgs a) {
       if (need != 0u) {
         const int q = __ffs(need) - 1;
         need &= need - 1u;
-        const double* v = T.prim64 + 12 * (int64_t)(first + q);
-        const d3 v0 = mk3(__ldg(v + 0), __ldg(v + 1), __ldg(v + 2));
-        const d3 v1 = mk3(__ldg(v + 3), __ldg(v + 4), __ldg(v + 5));
-        const d3 v2 = mk3(__ldg(v + 6), __ldg(v + 7), __ldg(v + 8));
-        const d3 v3 = mk3(__ldg(v + 9), __ldg(v + 10), __ldg(v + 11));
-        if (tet_contains64(p, v0, v1, v2, v3)) take(__ldg(&T.prim_ref[first + q]));
+        if (tet_contains64(p, T.prim64 + 12 * (int64_t)(first + q))) take(__ldg(&T.prim_ref[first + q]));
       }
     }
     if (leaf) pop();
