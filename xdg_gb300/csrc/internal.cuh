@@ -131,7 +131,7 @@ inline int device_sm_count() {
 // mixed closest of 1,000 points 584 -> 202 us, 8,000 576 -> 354, 30,011 683 ->
 // 566 (65,000 at 16 instead of 32: 1071 against 832); mixed find_element of
 // 1,000 60 -> 31 us; mixed ray_fire of 1,000 rays of the nested spheres 122 ->
-// 92 us, 20,000 147 -> 136; all-FP64 ray_fire of 5,000 rays 225 -> 187 us
+// 92 us, 20,000 147 -> 136; mixed find_volume of 20,000 points 312 -> 289; all-FP64 ray_fire of 5,000 rays 225 -> 187 us
 // (20,000 at 8: 278 against 227); all-FP64 closest of 1,000 3.29 -> 2.14 ms.
 constexpr int kSpreadWarps = 16, kFp64Warps = 6;
 inline int lanes_per_warp(int64_t n, int warps_per_sm) {

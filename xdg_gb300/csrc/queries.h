@@ -49,6 +49,7 @@ struct SurfArgs {
   int32_t occupancy;   // traversal kernel variant: minimum resident blocks per SM (2..4)
   int32_t width8;      // some surface tree has 8-wide nodes
   int32_t node_iters;  // inner-node steps per lane between leaf phases (1..64)
+  int32_t flush_queue; // queued candidates that force a drain (set by the launch)
   int32_t flush_wait;  // lanes waiting on the FP64 queue that force a partial drain (1..32)
   int32_t stack;       // shared-memory traversal stack entries per lane (16..64, multiple of 8)
   int32_t grab;        // > 0: warps take rays from the device work queue `work`, `grab` at a time

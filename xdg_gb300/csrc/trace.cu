@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(kTBlock, MINB) k_trace(SurfArgs a, int64_t chu
       const int qn = (int)(qtail - head);
       const unsigned act2 = __ballot_sync(kFull, trav);
       const unsigned waiting = __ballot_sync(kFull, has_ray && !trav && npend > 0);
-      if (!(qn >= 32 || (qn > 0 && (act2 == 0u || __popc(waiting) >= a.flush_wait)))) break;
+      if (!(qn >= a.flush_queue || (qn > 0 && (act2 == 0u || __popc(waiting) >= a.flush_wait)))) break;
       const int nq = min(qn, 32);
       const bool mine = lane < nq;
       const uint32_t ent = mine ? Q.ent[(head + lane) & (kQ - 1)] : ((uint32_t)lane << 27);
@@ -843,6 +843,27 @@ __global__ void __launch_bounds__(kTBlock, MINB) k_trace(SurfArgs a, int64_t chu
 std::atomic<int> g_blocks_per_sm[12][4][kTStackMax / 8 + 1][kMaxDevices];
 std::atomic<bool> g_smem_attr[12][4][kMaxDevices];
 
+// Queued candidates for which a warp drains its queue at once (1 .. 32).  A
+// drain costs the FP64 unit the same for one candidate as for 32, so full
+// batches wait for 32.  But until a ray's candidate has its exact distance the
+// ray is not cut short, and a point that restarts in volume after volume
+// carries that wait through each: the fewer rays a warp has, the sooner it
+// drains.  Nested spheres, draining at 32 / the rule's: find_volume of 1,000
+// points 365 / 132 us, 20,000 464 / 289, 1e5 680 / 529, 1e6 2.29 / 2.12 ms;
+// ray_fire of 1,000 rays 81 / 74 us, 20,000 119 / 113 (1e5 in the box at 4: 107
+// against 97); FP64 find_volume of 2,000 550 / 396 us; the FP64 particle loop of
+// 20,000 36.2 / 34.1 ms.
+int flush_queue_for(int mode, bool mixed, int64_t n, int lanes) {
+  const int64_t full = (int64_t)device_sm_count() * kSpreadWarps * 32;  // a ray for every lane
+  if (mode == MODE_FIND_VOLUME || mode == MODE_ALL_VOLUMES) {
+    if (!mixed) return n < full ? 4 : 32;
+    return n < full ? 1 : (n < 2 * full ? 4 : 12);
+  }
+  if (mode == MODE_PARTICLE) return mixed ? 32 : 12;
+  if (!mixed || n >= full) return 32;
+  return lanes <= 2 ? 1 : (lanes <= 8 ? 2 : 4);
+}
+
 template <int MODE, bool MIXED, int MINB, bool W8>
 cudaError_t launch_minb(const SurfArgs& a, cudaStream_t st, int slot) {
   constexpr int kVar = W8 ? MINB - 2 : 3;
@@ -866,11 +887,13 @@ cudaError_t launch_minb(const SurfArgs& a, cudaStream_t st, int slot) {
         occupancy_cached(g_blocks_per_sm[slot][kVar][a.stack / 8], kern, kTBlock, smem, per_sm);
     if (e != cudaSuccess) return e;
   }
-  // (a ray of these modes waits for memory; the rest wait for the FP64 unit,
-  // or restart in tree after tree, and do better with fuller warps)
-  constexpr bool spread = MIXED && (MODE == MODE_RAY_FIRE || MODE == MODE_PIV ||
-                                    MODE == MODE_OCCLUDED);
+  // (a ray of these modes waits for memory; the others wait for the FP64 unit
+  // and do better with fuller warps)
+  constexpr bool restarts = MODE == MODE_FIND_VOLUME || MODE == MODE_ALL_VOLUMES;
+  constexpr bool spread = restarts || (MIXED && MODE != MODE_PARTICLE);
   const int lanes = lanes_per_warp(a.n, spread ? kSpreadWarps : kFp64Warps);
+  SurfArgs b = a;
+  b.flush_queue = flush_queue_for(MODE, MIXED, a.n, lanes);
   const int64_t warps_needed = (a.n + lanes - 1) / lanes;
   int64_t blocks = (int64_t)device_sm_count() * per_sm;
   const int64_t max_blocks = (warps_needed + kTWarps - 1) / kTWarps;
@@ -878,7 +901,7 @@ cudaError_t launch_minb(const SurfArgs& a, cudaStream_t st, int slot) {
   if (blocks < 1) blocks = 1;
   const int64_t warps = blocks * kTWarps;
   const int64_t chunk = a.grab > 0 ? 0 : (a.n + warps - 1) / warps;
-  kern<<<(unsigned)blocks, kTBlock, smem, st>>>(a, chunk);
+  kern<<<(unsigned)blocks, kTBlock, smem, st>>>(b, chunk);
   return cudaGetLastError();
 }
 
