@@ -258,10 +258,10 @@ int xdgcu_walk_elements(xdgcu_ctx* ctx, int64_t n, const int32_t* start_index,
  * a track whose segments do not fit is not written and gets
  * XDGCU_RAY_OUTPUT_FULL (call again with capacity >= offsets[n]).  max_segs
  * caps the segments of one track (XDGCU_RAY_WALK_LIMIT).  Each track is
- * walked once, in rounds of walks capped at 16..256 segments per track: a
+ * walked once, in rounds of walks capped at 16..512 segments per track: a
  * walk that reaches the cap pauses and the next round resumes it where it
  * stopped; each round's segments wait in temporary device memory (about the
- * output's size, plus a buffer of up to 1 GiB, allocated on `stream` from
+ * output's size, plus a buffer of up to 4 GiB, allocated on `stream` from
  * the context's scratch pool, "scratch_keep_bytes") until the offsets are
  * known.  Where that memory cannot be
  * had, or with the tuning key "packed_walk_passes" = 2, the tracks are walked
@@ -292,8 +292,8 @@ int xdgcu_set_boundary_face_elements(xdgcu_ctx* ctx, int64_t n, const int32_t* f
  * together: each round is one find_element launch for the tracks to locate,
  * one ray_fire launch for those outside the mesh and one walk launch, with
  * the bookkeeping in device kernels.  A round's walk emits at most K
- * segments per track (K = 16..256, chosen so the round buffer stays near
- * 1 GiB); a longer walk pauses and the next round resumes it from where it
+ * segments per track (K = 16..512, chosen so the round buffer stays near
+ * 4 GiB); a longer walk pauses and the next round resumes it from where it
  * stopped, with the same operations as one uninterrupted walk.
  * Output as xdgcu_walk_elements_packed: track i's segments (element MESH
  * ids, lengths) at offsets[i] .. offsets[i+1]-1 of arrays of `capacity`
@@ -595,8 +595,8 @@ int xdgcu_get_counters(xdgcu_ctx* ctx, int64_t counters[8]);
  *   "segments_walk_cap"  xdgcu_segments_global and the packed walk's rounds:
  *                      segments a walk emits per
  *                      round before it pauses (1..1024; 0, the default, picks
- *                      per round the largest power of two in 16..256 for which
- *                      that round's walks fit a buffer of about 1 GiB, so
+ *                      per round the largest power of two in 16..512 for which
+ *                      that round's walks fit a buffer of about 4 GiB, so
  *                      rounds with fewer walks pause fewer of them).  Results
  *                      do not depend on it
  *   "walk_edge_table"  walk: 1 (default) takes the FP64 Plucker

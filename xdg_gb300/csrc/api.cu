@@ -1176,9 +1176,12 @@ struct CallScratch {
   }
 };
 
-// The K-strided walk buffer of xdgcu_segments_global (12 bytes per slot)
-// holds at most about this many bytes.
-constexpr int64_t kSegStridedBytes = int64_t(1) << 30;
+// The K-strided walk buffer of the rounds (12 bytes per slot) holds at most
+// about this many bytes, or kSegStridedLeast where those cannot be had.  A
+// round that pauses no walk needs neither a second length order nor a second
+// end (1e6 tracks located and walked: 7.56 ms with 1 GiB, 7.16 with 4).
+constexpr int64_t kSegStridedBytes = int64_t(4) << 30;
+constexpr int64_t kSegStridedLeast = int64_t(1) << 30;
 
 // D2H of one counter, waited for.
 cudaError_t read_count(const int32_t* d, int32_t* h, cudaStream_t st) {
@@ -1189,15 +1192,15 @@ cudaError_t read_count(const int32_t* d, int32_t* h, cudaStream_t st) {
 
 // Rounds of single-pass walks (the global track loop and the packed walk):
 // the K-strided buffer of n tracks holds seg_strided_cap entries, about
-// kSegStridedBytes (at least 16 per track, 256 at most), or fixed_k per track
-// when that is set; a round of `walks` walks takes the largest K <= 256 (a
-// power of two) that fits, so rounds with fewer walks pause fewer of them.
-int64_t seg_strided_cap(int64_t n, int64_t fixed_k) {
+// `bytes` (at least 16 per track, 512 at most), or fixed_k per track when that
+// is set; a round of `walks` walks takes the largest K <= 512 (a power of two)
+// that fits, so rounds with fewer walks pause fewer of them.
+int64_t seg_strided_cap(int64_t n, int64_t fixed_k, int64_t bytes) {
   return fixed_k > 0 ? fixed_k * n
-                     : std::max<int64_t>(16 * n, std::min<int64_t>(256 * n, kSegStridedBytes / 12));
+                     : std::max<int64_t>(16 * n, std::min<int64_t>(512 * n, bytes / 12));
 }
 int32_t seg_round_k(int64_t walks, int64_t cap, int64_t fixed_k, int32_t max_segs) {
-  int32_t K = (int32_t)(fixed_k > 0 ? fixed_k : 256);
+  int32_t K = (int32_t)(fixed_k > 0 ? fixed_k : 512);
   while (fixed_k <= 0 && K > 16 && (int64_t)K * walks > cap) K >>= 1;
   return std::min(K, max_segs);
 }
@@ -1221,6 +1224,19 @@ struct SegWalkBufs {
   double *wr, *wu, *wd, *wsum_in, *wsum_out, *wend_r, *wend_d, *sk_len;
   int64_t strided_cap;
 };
+
+// The K-strided buffer of n tracks, with less where the memory is short.
+cudaError_t seg_strided_alloc(const xdgcu_ctx* c, int64_t n, CallScratch& S, SegWalkBufs& B) {
+  cudaError_t e = cudaSuccess;
+  for (int64_t bytes : {kSegStridedBytes, kSegStridedLeast}) {
+    B.strided_cap = seg_strided_cap(n, c->segments_walk_cap, bytes);
+    e = S.get(&B.sk_len, B.strided_cap);
+    if (e == cudaSuccess) e = S.get(&B.sk_elem, B.strided_cap);
+    if (e == cudaSuccess) return e;
+    cudaGetLastError();  // the failed allocation is not a pending launch error
+  }
+  return e;
+}
 
 // One round of the capped single-pass walk for the m entries of the walk
 // list: walk_elements from each track's walk state, at most K segments per
@@ -1346,9 +1362,10 @@ int walk_packed_rounds(xdgcu_ctx* c, bool mixed, const WalkArgs& a, cudaStream_t
   get(&B.wsum_out, n);
   get(&B.wend_r, 3 * n);
   get(&B.wend_d, n);
-  B.strided_cap = seg_strided_cap(n, c->segments_walk_cap);
-  get(&B.sk_elem, B.strided_cap);
-  get(&B.sk_len, B.strided_cap);
+  if (ok && seg_strided_alloc(c, n, S, B) != cudaSuccess) {
+    ok = false;
+    *no_memory = true;
+  }
   if (!ok) return set_err(XDGCU_ERR_CUDA, "walk_elements_packed: temporary memory");
   int32_t* n_act = counters;
   int32_t* n_walk = counters + 1;
@@ -2731,7 +2748,6 @@ int xdgcu_segments_global(xdgcu_ctx* c, int32_t ipc_tree, int32_t element_tree, 
   API_CUDA(S.get(&t_hit, n), "segments scratch");
   // the walk list and the rounds' walk buffers (seg_walk_round)
   SegWalkBufs B{};
-  B.strided_cap = seg_strided_cap(n, c->segments_walk_cap);
   API_CUDA(S.get(&B.walk_t, n), "segments scratch");
   API_CUDA(S.get(&B.walk_start, n), "segments scratch");
   API_CUDA(S.get(&B.wst, n), "segments scratch");
@@ -2744,8 +2760,7 @@ int xdgcu_segments_global(xdgcu_ctx* c, int32_t ipc_tree, int32_t element_tree, 
   API_CUDA(S.get(&B.wsum_out, n), "segments scratch");
   API_CUDA(S.get(&B.wend_r, 3 * n), "segments scratch");
   API_CUDA(S.get(&B.wend_d, n), "segments scratch");
-  API_CUDA(S.get(&B.sk_elem, B.strided_cap), "segments scratch");
-  API_CUDA(S.get(&B.sk_len, B.strided_cap), "segments scratch");
+  API_CUDA(seg_strided_alloc(c, n, S, B), "segments scratch");
   int32_t* n_act = counters;
   int32_t* n_walk = counters + 1;
   int32_t* n_out = counters + 2;

@@ -151,22 +151,32 @@ __device__ __forceinline__ bool in_range3(d3 v) {
   return in_range(v.x) && in_range(v.y) && in_range(v.z);
 }
 
-__device__ __forceinline__ double dot3_i(d3 a, d3 b) {
-  return mul_int(a.x, b.x) + mul_int(a.y, b.y) + mul_int(a.z, b.z);
+// a * b on the integer pipes (INT) or the FP64 unit
+template <bool INT>
+__device__ __forceinline__ double mul_p(double a, double b) {
+  return INT ? mul_int(a, b) : a * b;
 }
 
-__device__ __forceinline__ d3 cross3_i(d3 a, d3 b) {
-  return mk3(mul_int(a.y, b.z) - mul_int(a.z, b.y), mul_int(a.z, b.x) - mul_int(a.x, b.z),
-             mul_int(a.x, b.y) - mul_int(a.y, b.x));
+template <bool INT>
+__device__ __forceinline__ double dot3_p(d3 a, d3 b) {
+  return mul_p<INT>(a.x, b.x) + mul_p<INT>(a.y, b.y) + mul_p<INT>(a.z, b.z);
+}
+
+template <bool INT>
+__device__ __forceinline__ d3 cross3_p(d3 a, d3 b) {
+  return mk3(mul_p<INT>(a.y, b.z) - mul_p<INT>(a.z, b.y),
+             mul_p<INT>(a.z, b.x) - mul_p<INT>(a.x, b.z),
+             mul_p<INT>(a.x, b.y) - mul_p<INT>(a.y, b.x));
 }
 
 // plucker_edge_pre for a reference of edge_ref()
-__device__ __forceinline__ double edge_coord_i(const double* edge, int32_t ref, d3 u, d3 rn) {
+template <bool INT>
+__device__ __forceinline__ double edge_coord_p(const double* edge, int32_t ref, d3 u, d3 rn) {
   const double* E = edge + 6 * (int64_t)(ref & 0x7fffffff);
   const double2 a = __ldg(reinterpret_cast<const double2*>(E));
   const double2 b = __ldg(reinterpret_cast<const double2*>(E + 2));
   const double2 c = __ldg(reinterpret_cast<const double2*>(E + 4));
-  double pip = dot3_i(u, mk3(b.y, c.x, c.y)) + dot3_i(rn, mk3(a.x, a.y, b.x));
+  double pip = dot3_p<INT>(u, mk3(b.y, c.x, c.y)) + dot3_p<INT>(rn, mk3(a.x, a.y, b.x));
   pip = __longlong_as_double(__double_as_longlong(pip) ^ ((long long)(ref & 0x80000000) << 32));
   if (absbits(pip) < absbits(ZERO_TOL)) pip = 0.0;
   return pip;
@@ -179,18 +189,19 @@ __device__ __noinline__ bool sum_above_one(double a, double b) { return dlt(1.0,
 // or INFTY for no hit.  The weights are >= 0, and their sum is tested only
 // where it can exceed 1: w1 >= 2^-48 keeps w0 + w2 below 1, since the
 // weights' sum is within 6 eps of 1.
-__device__ __forceinline__ double face_distance_i(double c0, double c1, double c2, double v0i,
+template <bool INT>
+__device__ __forceinline__ double face_distance_p(double c0, double c1, double c2, double v0i,
                                                   double v1i, double v2i, double oi, double di) {
   const double inv = 1.0 / (c0 + c1 + c2);
-  const double w0 = mul_int(c0, inv), w1 = mul_int(c1, inv), w2 = mul_int(c2, inv);
-  const double hit = (mul_int(w0, v2i) + mul_int(w1, v0i)) + mul_int(w2, v1i);
+  const double w0 = mul_p<INT>(c0, inv), w1 = mul_p<INT>(c1, inv), w2 = mul_p<INT>(c2, inv);
+  const double hit = (mul_p<INT>(w0, v2i) + mul_p<INT>(w1, v0i)) + mul_p<INT>(w2, v1i);
   double t = (hit - oi) / di;
   if (absbits(w1) < 0x3cf0000000000000ull && sum_above_one(w2, w0)) t = -1.0;
   if (lt0(t) || dlt(INFTY, t)) return INFTY;
   return gt0(t) ? t : 0.0;
 }
 
-// The exit distance through one face, as face_distance_i, from the edge
+// The exit distance through one face, as face_distance_p, from the edge
 // table with the products on the FP64 unit: edge references e0..e2 of
 // edge_ref(), vertex indices i0..i2.
 __device__ __noinline__ double face_exit_hw(const double* edge, const double* xyz, int32_t e0,
@@ -251,7 +262,8 @@ __device__ __forceinline__ StepDir step_dir(const WalkArgs& a, d3 u) {
 
 // MeshManager::next_element for the tet of record T at r along u.  Returns the face
 // index (or -1) and writes the exit distance.
-template <int FO, bool MIXED>
+// INT: the products of a safe step run on the integer pipes.
+template <int FO, bool MIXED, bool INT = true>
 __device__ __forceinline__ int next_face(const WalkArgs& a, const TetRec& T, d3 r, d3 u,
                                          const StepDir& sd, bool safe, double* exit_dist,
                                          StepCnt& cnt) {
@@ -261,7 +273,7 @@ __device__ __forceinline__ int next_face(const WalkArgs& a, const TetRec& T, d3 
   unsigned escm = 0u;
   d3 rn = mk3(0.0, 0.0, 0.0);
   double pe[6];  // FP64 path: the six coordinates, pair (i, j), i < j, run i -> j
-  if (safe) rn = cross3_i(u, r);  // plucker.h:75
+  if (safe) rn = cross3_p<INT>(u, r);  // plucker.h:75
   if (!MIXED) {
     escm = 0xfu;
     if (safe) {
@@ -270,7 +282,7 @@ __device__ __forceinline__ int next_face(const WalkArgs& a, const TetRec& T, d3 
       for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = i + 1; j < 4; ++j)
-          pe[pair_index(i, j)] = edge_coord_i(a.edge, edge_ref(te, i, j), u, rn);
+          pe[pair_index(i, j)] = edge_coord_p<INT>(a.edge, edge_ref(te, i, j), u, rn);
 #pragma unroll
       for (int f = 0; f < 4; ++f) {
         const int l[3] = {face_local<FO>(a, f, 0), face_local<FO>(a, f, 1),
@@ -351,9 +363,9 @@ __device__ __forceinline__ int next_face(const WalkArgs& a, const TetRec& T, d3 
     if (safe) {
       double c0, c1, c2;
       if (MIXED) {
-        c0 = edge_coord_i(a.edge, edge_ref(te, l0, l1), u, rn);
-        c1 = edge_coord_i(a.edge, edge_ref(te, l1, l2), u, rn);
-        c2 = edge_coord_i(a.edge, edge_ref(te, l2, l0), u, rn);
+        c0 = edge_coord_p<INT>(a.edge, edge_ref(te, l0, l1), u, rn);
+        c1 = edge_coord_p<INT>(a.edge, edge_ref(te, l1, l2), u, rn);
+        c2 = edge_coord_p<INT>(a.edge, edge_ref(te, l2, l0), u, rn);
       } else {
         // (negated where the face runs the pair backwards; 0 stays +0)
         auto coord = [&](int la, int lb) {
@@ -365,7 +377,7 @@ __device__ __forceinline__ int next_face(const WalkArgs& a, const TetRec& T, d3 
         c2 = coord(l2, l0);
       }
       if (!(gt0(c0) || gt0(c1) || gt0(c2)) && !(is0(c0) && is0(c1) && is0(c2)))
-        df = face_distance_i(c0, c1, c2, __ldg(&a.xyz[3 * (int64_t)i0 + sd.axis]),
+        df = face_distance_p<INT>(c0, c1, c2, __ldg(&a.xyz[3 * (int64_t)i0 + sd.axis]),
                              __ldg(&a.xyz[3 * (int64_t)i1 + sd.axis]),
                              __ldg(&a.xyz[3 * (int64_t)i2 + sd.axis]), comp3(r, sd.axis),
                              comp3(u, sd.axis));
@@ -454,8 +466,9 @@ struct WarpTracks {
 // a warp keeps all 32 lanes stepping until its tracks are used up (track
 // lengths are exponentially distributed, so one-track-per-lane would leave
 // most lanes idle behind the longest track of the warp).
-// SUM: the running length sum is wanted (WalkArgs::sum_out).
-template <int FO, bool MIXED, bool SUM>
+// SUM: the running length sum is wanted (WalkArgs::sum_out).  INT: products on
+// the integer pipes (next_face).
+template <int FO, bool MIXED, bool SUM, bool INT>
 __global__ void __launch_bounds__(kBlock, 4) k_walk(WalkArgs a, int64_t chunk) {
   const int lane = threadIdx.x & 31;
   const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -527,7 +540,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(WalkArgs a, int64_t chunk) {
         double ex;
         const TetRec T = load_rec(a, elem);
         const bool safe = sd.safe && in_range3(r);
-        const int f = next_face<FO, MIXED>(a, T, r, u, sd, safe, &ex, cnt);
+        const int f = next_face<FO, MIXED, INT>(a, T, r, u, sd, safe, &ex, cnt);
         int32_t nxt = -1;
         if (f < 0) {
           st = RAY_NO_EXIT_FACE;  // the reference would index adjacency with -1
@@ -1011,10 +1024,10 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_apply(int64_t* __restrict__
   if (blockIdx.x == 0 && threadIdx.x == 0) v[n] = sums[nb];
 }
 
-template <int FO, bool MIXED, bool QUEUE, bool SUM>
+template <int FO, bool MIXED, bool QUEUE, bool SUM, bool INT = true>
 cudaError_t launch_walk_s(const WalkArgs& a, cudaStream_t st) {
   static std::atomic<int> cached[kMaxDevices];  // resident blocks per SM, per device
-  auto kern = QUEUE ? k_walk_q<FO> : k_walk<FO, MIXED, SUM>;
+  auto kern = QUEUE ? k_walk_q<FO> : k_walk<FO, MIXED, SUM, INT>;
   int per_sm = 0;
   const cudaError_t e = occupancy_cached(cached, kern, kBlock, 0, per_sm);
   if (e != cudaSuccess) return e;
@@ -1035,6 +1048,13 @@ cudaError_t launch_walk_s(const WalkArgs& a, cudaStream_t st) {
 
 template <int FO, bool MIXED, bool QUEUE>
 cudaError_t launch_walk_t(const WalkArgs& a, cudaStream_t st) {
+  // With at most about one warp a scheduler a step is a chain, and in the
+  // all-FP64 step, with 45 products, the FP64 unit's are the shorter links
+  // (1,000 tracks located and walked 2.11 ms with the integer products, 1.84
+  // without; 20,000 3.25 and 2.49; 60,000 3.71 and 4.27)
+  if (!MIXED && a.n <= (int64_t)device_sm_count() * kFp64Warps * 32)
+    return a.sum_out ? launch_walk_s<FO, MIXED, QUEUE, true, MIXED>(a, st)
+                     : launch_walk_s<FO, MIXED, QUEUE, false, MIXED>(a, st);
   return a.sum_out ? launch_walk_s<FO, MIXED, QUEUE, true>(a, st)
                    : launch_walk_s<FO, MIXED, QUEUE, false>(a, st);
 }
