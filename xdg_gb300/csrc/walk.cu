@@ -30,6 +30,7 @@
 // FP64 evaluation error and the 20*DBL_EPSILON snap are added as in geom.cuh).
 #include "walk.h"
 
+#include <algorithm>
 #include <atomic>
 
 #include <cub/device/device_radix_sort.cuh>
@@ -184,23 +185,6 @@ __device__ __forceinline__ double edge_coord_p(const double* edge, int32_t ref, 
 
 __device__ __noinline__ bool sum_above_one(double a, double b) { return dlt(1.0, a + b); }
 
-// plucker64_coords for the walk's call (orientation +1, distances 0 ..
-// INFTY), for coordinates that are all <= 0 and not all 0: max(0, distance),
-// or INFTY for no hit.  The weights are >= 0, and their sum is tested only
-// where it can exceed 1: w1 >= 2^-48 keeps w0 + w2 below 1, since the
-// weights' sum is within 6 eps of 1.
-template <bool INT>
-__device__ __forceinline__ double face_distance_p(double c0, double c1, double c2, double v0i,
-                                                  double v1i, double v2i, double oi, double di) {
-  const double inv = 1.0 / (c0 + c1 + c2);
-  const double w0 = mul_p<INT>(c0, inv), w1 = mul_p<INT>(c1, inv), w2 = mul_p<INT>(c2, inv);
-  const double hit = (mul_p<INT>(w0, v2i) + mul_p<INT>(w1, v0i)) + mul_p<INT>(w2, v1i);
-  double t = (hit - oi) / di;
-  if (absbits(w1) < 0x3cf0000000000000ull && sum_above_one(w2, w0)) t = -1.0;
-  if (lt0(t) || dlt(INFTY, t)) return INFTY;
-  return gt0(t) ? t : 0.0;
-}
-
 // The exit distance through one face, as face_distance_p, from the edge
 // table with the products on the FP64 unit: edge references e0..e2 of
 // edge_ref(), vertex indices i0..i2.
@@ -260,29 +244,110 @@ __device__ __forceinline__ StepDir step_dir(const WalkArgs& a, d3 u) {
   return s;
 }
 
+// Lanes of a track.  G = 4: four neighbouring lanes hold the same track and go
+// the same way; in a safe step they share its independent values (a component
+// of u x r, an edge's coordinate, a weight) and hand them round.  A step of a
+// lone warp is a chain of some 1,900 instructions and 43 FP64 ones, 32 lanes
+// wide or one; shared it is two thirds of that, for a quarter of the tracks a
+// warp, so small batches walk this way (kTeamWarps).  1,000 tracks located and
+// walked: mixed 1.34 -> 1.10 ms, all-FP64 1.85 -> 1.35; 1,000 particles of the
+// walk_elements loop 6.0 -> 5.1 ms.
+template <int G>
+struct Team {
+  unsigned mask;
+  int q;  // the lane's place in its team
+  __device__ __forceinline__ Team() {
+    const int lane = threadIdx.x & 31;
+    q = G > 1 ? lane & (G - 1) : 0;
+    mask = G > 1 ? ((1u << G) - 1u) << (lane & ~(G - 1)) : 0u;
+  }
+  __device__ __forceinline__ double from(double v, int place) const {
+    return G > 1 ? __shfl_sync(mask, v, place, G) : v;
+  }
+  __device__ __forceinline__ d3 gather(double v) const {
+    return mk3(from(v, 0), from(v, 1), from(v, 2));
+  }
+};
+
+// plucker64_coords for the walk's call (orientation +1, distances 0 ..
+// INFTY), for coordinates that are all <= 0 and not all 0: max(0, distance),
+// or INFTY for no hit.  The weights are >= 0, and their sum is tested only
+// where it can exceed 1: w1 >= 2^-48 keeps w0 + w2 below 1, since the
+// weights' sum is within 6 eps of 1.
+template <bool INT, int G>
+__device__ __forceinline__ double face_distance_p(const Team<G>& team, double c0, double c1,
+                                                  double c2, const double* xyz, int32_t i0,
+                                                  int32_t i1, int32_t i2, double oi, double di) {
+  // (xyz: the vertices' components along plucker_axis)
+  auto comp = [&](int32_t i) { return __ldg(&xyz[3 * (int64_t)i]); };
+  const double inv = 1.0 / (c0 + c1 + c2);
+  double w0, w1, w2, hit;
+  if (G == 1) {
+    w0 = mul_p<INT>(c0, inv);
+    w1 = mul_p<INT>(c1, inv);
+    w2 = mul_p<INT>(c2, inv);
+    hit = (mul_p<INT>(w0, comp(i2)) + mul_p<INT>(w1, comp(i0))) + mul_p<INT>(w2, comp(i1));
+  } else {
+    const int k = team.q == 3 ? 0 : team.q;
+    const double w = mul_p<INT>(k == 0 ? c0 : (k == 1 ? c1 : c2), inv);
+    const d3 p = team.gather(mul_p<INT>(w, comp(k == 0 ? i2 : (k == 1 ? i0 : i1))));
+    w0 = team.from(w, 0);
+    w1 = team.from(w, 1);
+    w2 = team.from(w, 2);
+    hit = (p.x + p.y) + p.z;
+  }
+  double t = (hit - oi) / di;
+  if (absbits(w1) < 0x3cf0000000000000ull && sum_above_one(w2, w0)) t = -1.0;
+  if (lt0(t) || dlt(INFTY, t)) return INFTY;
+  return gt0(t) ? t : 0.0;
+}
+
+template <int G>
+__device__ __forceinline__ d3 walk_move(const Team<G>& team, d3 r, double len, d3 u) {
+  if (G == 1) return add3(r, scl3(len, u));
+  const int k = team.q == 3 ? 0 : team.q;
+  return team.gather(comp3(r, k) + len * comp3(u, k));
+}
+
 // MeshManager::next_element for the tet of record T at r along u.  Returns the face
 // index (or -1) and writes the exit distance.
 // INT: the products of a safe step run on the integer pipes.
-template <int FO, bool MIXED, bool INT = true>
+template <int FO, bool MIXED, bool INT = true, int G = 1>
 __device__ __forceinline__ int next_face(const WalkArgs& a, const TetRec& T, d3 r, d3 u,
                                          const StepDir& sd, bool safe, double* exit_dist,
-                                         StepCnt& cnt) {
+                                         StepCnt& cnt, const Team<G>& team = Team<G>()) {
   const int32_t* ci = T.v;
   const int32_t* te = T.edge;
+  const int tq = team.q == 3 ? 0 : team.q;  // the value of three that this lane evaluates
   // the faces that may be the exit face: only these take the distance below
   unsigned escm = 0u;
   d3 rn = mk3(0.0, 0.0, 0.0);
   double pe[6];  // FP64 path: the six coordinates, pair (i, j), i < j, run i -> j
-  if (safe) rn = cross3_p<INT>(u, r);  // plucker.h:75
+  if (safe) {  // plucker.h:75
+    if (G == 1) {
+      rn = cross3_p<INT>(u, r);
+    } else {
+      const int k1 = tq == 2 ? 0 : tq + 1, k2 = tq == 0 ? 2 : tq - 1;
+      rn = team.gather(mul_p<INT>(comp3(u, k1), comp3(r, k2)) -
+                       mul_p<INT>(comp3(u, k2), comp3(r, k1)));
+    }
+  }
   if (!MIXED) {
     escm = 0xfu;
     if (safe) {
       escm = 0u;
+      // (a record's own references run their pairs i -> j)
+      if (G == 1) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+        for (int k = 0; k < 6; ++k) pe[k] = edge_coord_p<INT>(a.edge, te[k], u, rn);
+      } else {
+        const double p = edge_coord_p<INT>(a.edge, sel4(te, team.q), u, rn);
+        const double p4 = edge_coord_p<INT>(a.edge, (team.q & 1) ? te[5] : te[4], u, rn);
 #pragma unroll
-        for (int j = i + 1; j < 4; ++j)
-          pe[pair_index(i, j)] = edge_coord_p<INT>(a.edge, edge_ref(te, i, j), u, rn);
+        for (int k = 0; k < 4; ++k) pe[k] = team.from(p, k);
+        pe[4] = team.from(p4, 0);
+        pe[5] = team.from(p4, 1);
+      }
 #pragma unroll
       for (int f = 0; f < 4; ++f) {
         const int l[3] = {face_local<FO>(a, f, 0), face_local<FO>(a, f, 1),
@@ -362,7 +427,13 @@ __device__ __forceinline__ int next_face(const WalkArgs& a, const TetRec& T, d3 
     double df = INFTY;
     if (safe) {
       double c0, c1, c2;
-      if (MIXED) {
+      if (MIXED && G > 1) {
+        const int la = tq == 0 ? l0 : (tq == 1 ? l1 : l2), lb = tq == 0 ? l1 : (tq == 1 ? l2 : l0);
+        const d3 c = team.gather(edge_coord_p<INT>(a.edge, edge_ref(te, la, lb), u, rn));
+        c0 = c.x;
+        c1 = c.y;
+        c2 = c.z;
+      } else if (MIXED) {
         c0 = edge_coord_p<INT>(a.edge, edge_ref(te, l0, l1), u, rn);
         c1 = edge_coord_p<INT>(a.edge, edge_ref(te, l1, l2), u, rn);
         c2 = edge_coord_p<INT>(a.edge, edge_ref(te, l2, l0), u, rn);
@@ -377,10 +448,8 @@ __device__ __forceinline__ int next_face(const WalkArgs& a, const TetRec& T, d3 
         c2 = coord(l2, l0);
       }
       if (!(gt0(c0) || gt0(c1) || gt0(c2)) && !(is0(c0) && is0(c1) && is0(c2)))
-        df = face_distance_p<INT>(c0, c1, c2, __ldg(&a.xyz[3 * (int64_t)i0 + sd.axis]),
-                             __ldg(&a.xyz[3 * (int64_t)i1 + sd.axis]),
-                             __ldg(&a.xyz[3 * (int64_t)i2 + sd.axis]), comp3(r, sd.axis),
-                             comp3(u, sd.axis));
+        df = face_distance_p<INT, G>(team, c0, c1, c2, a.xyz + sd.axis, i0, i1, i2,
+                                     comp3(r, sd.axis), comp3(u, sd.axis));
     } else if (a.edge) {
       df = face_exit_hw(a.edge, a.xyz, edge_ref(te, l0, l1), edge_ref(te, l1, l2),
                         edge_ref(te, l2, l0), i0, i1, i2, r, u);
@@ -425,14 +494,16 @@ __device__ __forceinline__ void walk_end_state(const WalkArgs& a, int64_t i, d3 
 
 // Where a warp's tracks come from: positions cursor .. end - 1 of the batch,
 // or of the length order.  Without an order, one contiguous chunk.  With one,
-// the warp takes 32 consecutive positions at a time, longest first, from the
+// the warp takes 32 (eight teams: 8) consecutive positions at a time, longest first, from the
 // launch's work counter.  The lanes of a warp then hold tracks of about the
 // same length and end together, so the FP64 unit, which takes as long for one
 // lane as for 32, sees full warps (dealt one by one, every warp held one of
 // the longest tracks and stepped on for it alone), and the warps end together
 // too (dealt in fixed shares, the SMs were idle a fifth of the launch on
 // 3e5 tracks).
+template <int G = 1>
 struct WarpTracks {
+  static constexpr int kTake = 32 / G;  // tracks a warp holds
   int64_t cursor, end;
   __device__ __forceinline__ WarpTracks(const WalkArgs& a, int64_t gwarp, int64_t chunk) {
     cursor = a.order ? 0 : gwarp * chunk;
@@ -446,11 +517,11 @@ struct WarpTracks {
   __device__ __forceinline__ int64_t take(const WalkArgs& a, int rank, int want) {
     if (a.order && cursor >= end && end <= a.n) {
       unsigned long long base = 0ull;
-      if ((threadIdx.x & 31) == 0) base = atomicAdd(a.work, 32ull);
+      if ((threadIdx.x & 31) == 0) base = atomicAdd(a.work, (unsigned long long)kTake);
       base = __shfl_sync(0xffffffffu, base, 0);
       cursor = (int64_t)base;
       // (end stays past n once the order is used up, and no more is taken)
-      end = cursor < a.n ? min(a.n, cursor + 32) : a.n + 1;
+      end = cursor < a.n ? min(a.n, cursor + kTake) : a.n + 1;
       if (cursor >= a.n) cursor = end;
     }
     const int64_t pos = cursor + rank;
@@ -468,11 +539,12 @@ struct WarpTracks {
 // most lanes idle behind the longest track of the warp).
 // SUM: the running length sum is wanted (WalkArgs::sum_out).  INT: products on
 // the integer pipes (next_face).
-template <int FO, bool MIXED, bool SUM, bool INT>
+// G: lanes of a track (Team).
+template <int FO, bool MIXED, bool SUM, bool INT, int G>
 __global__ void __launch_bounds__(kBlock, 4) k_walk(WalkArgs a, int64_t chunk) {
-  const int lane = threadIdx.x & 31;
+  const Team<G> team;
   const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  WarpTracks list(a, gwarp, chunk);
+  WarpTracks<G> list(a, gwarp, chunk);
   StepCnt cnt = {0, 0};
   unsigned long long tracks = 0;
   bool has = false;
@@ -488,7 +560,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(WalkArgs a, int64_t chunk) {
     if (need != 0u) {
       unsigned lt;
       asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-      const int64_t cand = list.take(a, __popc(need & lt), __popc(need));
+      if (G > 1) lt = (1u << (threadIdx.x & 31 & ~(G - 1))) - 1u;
+      const int64_t cand = list.take(a, __popc(need & lt) / G, __popc(need) / G);
       if (!has) {
         if (cand >= 0) {
           i = cand;
@@ -536,11 +609,11 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(WalkArgs a, int64_t chunk) {
         done = true;
       }
       if (!done) {
-        cnt.steps++;
+        if (team.q == 0) cnt.steps++;
         double ex;
         const TetRec T = load_rec(a, elem);
         const bool safe = sd.safe && in_range3(r);
-        const int f = next_face<FO, MIXED, INT>(a, T, r, u, sd, safe, &ex, cnt);
+        const int f = next_face<FO, MIXED, INT, G>(a, T, r, u, sd, safe, &ex, cnt, team);
         int32_t nxt = -1;
         if (f < 0) {
           st = RAY_NO_EXIT_FACE;  // the reference would index adjacency with -1
@@ -550,12 +623,12 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(WalkArgs a, int64_t chunk) {
         ex = dlt(dist, ex) ? dist : ex;  // std::min(exit, distance)
         dist -= ex;
         if (SUM) sum = sum + ex;
-        if (oe) {
+        if (oe && team.q == 0) {
           oe[k] = T.id;
           ol[k] = ex;
         }
         ++k;
-        r = add3(r, scl3(ex, u));  // r += exit.second * u
+        r = walk_move(team, r, ex, u);  // r += exit.second * u
         if (nxt < -1 || nxt >= a.n_tets) {
           st = RAY_INVALID;  // corrupt adjacency: stop instead of reading out of range
           done = true;
@@ -564,7 +637,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(WalkArgs a, int64_t chunk) {
           if (elem == -1) done = true;
         }
       }
-      if (done) {
+      if (done) has = false;
+      if (done && team.q == 0) {
         if (a.out_mode == WALK_COUNT) {
           a.offsets[i] = k;
         } else {
@@ -574,7 +648,6 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(WalkArgs a, int64_t chunk) {
         if (a.status) a.status[i] = st;
         if (a.stop_elem) a.stop_elem[i] = elem;  // where a capped walk resumes
         walk_end_state(a, i, r, dist, sum);
-        has = false;
         tracks++;
       }
     }
@@ -694,7 +767,7 @@ __global__ void __launch_bounds__(kBlock) k_walk_q(WalkArgs a, int64_t chunk) {
   WalkQueue& Q = qs[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  WarpTracks list(a, gwarp, chunk);
+  WarpTracks<> list(a, gwarp, chunk);
   if (lane == 0) {
     Q.head = 0u;
     Q.tail = 0u;
@@ -1024,15 +1097,15 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_apply(int64_t* __restrict__
   if (blockIdx.x == 0 && threadIdx.x == 0) v[n] = sums[nb];
 }
 
-template <int FO, bool MIXED, bool QUEUE, bool SUM, bool INT = true>
+template <int FO, bool MIXED, bool QUEUE, bool SUM, bool INT = true, int G = 1>
 cudaError_t launch_walk_s(const WalkArgs& a, cudaStream_t st) {
   static std::atomic<int> cached[kMaxDevices];  // resident blocks per SM, per device
-  auto kern = QUEUE ? k_walk_q<FO> : k_walk<FO, MIXED, SUM, INT>;
+  auto kern = QUEUE ? k_walk_q<FO> : k_walk<FO, MIXED, SUM, INT, G>;
   int per_sm = 0;
   const cudaError_t e = occupancy_cached(cached, kern, kBlock, 0, per_sm);
   if (e != cudaSuccess) return e;
   int64_t blocks = (int64_t)device_sm_count() * per_sm;
-  const int lanes = a.order ? 32 : lanes_per_warp(a.n, kFp64Warps);
+  const int lanes = a.order ? 32 / G : std::min(32 / G, lanes_per_warp(a.n, kFp64Warps));
   const int64_t max_blocks = ((a.n + lanes - 1) / lanes + kBlock / 32 - 1) / (kBlock / 32);
   if (blocks > max_blocks) blocks = max_blocks;
   if (blocks < 1) blocks = 1;
@@ -1046,12 +1119,23 @@ cudaError_t launch_walk_s(const WalkArgs& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+// Warps of eight four-lane tracks per SM up to which a batch walks that way
+// (24,320 tracks): ms at 14 / 20 / 28, mixed: tally of 22,000 tracks 1.93 / 1.62 /
+// 1.61, 34,000 1.94 / 1.92 / 1.64; global tracks, whose rounds shrink, 22,000
+// 3.44 / 3.30 / 3.32, 60,000 4.07 / 4.07 / 4.24.
+constexpr int kTeamWarps = 20;
+
 template <int FO, bool MIXED, bool QUEUE>
 cudaError_t launch_walk_t(const WalkArgs& a, cudaStream_t st) {
   // With at most about one warp a scheduler a step is a chain, and in the
   // all-FP64 step, with 45 products, the FP64 unit's are the shorter links
   // (1,000 tracks located and walked 2.11 ms with the integer products, 1.84
   // without; 20,000 3.25 and 2.49; 60,000 3.71 and 4.27)
+  const int64_t team_max = (int64_t)device_sm_count() * kTeamWarps * 8;
+  if constexpr (FO == 0 && !QUEUE)
+    if (a.n <= team_max)
+      return a.sum_out ? launch_walk_s<FO, MIXED, false, true, MIXED, 4>(a, st)
+                       : launch_walk_s<FO, MIXED, false, false, MIXED, 4>(a, st);
   if (!MIXED && a.n <= (int64_t)device_sm_count() * kFp64Warps * 32)
     return a.sum_out ? launch_walk_s<FO, MIXED, QUEUE, true, MIXED>(a, st)
                      : launch_walk_s<FO, MIXED, QUEUE, false, MIXED>(a, st);
@@ -1094,9 +1178,11 @@ namespace {
 // many lanes at once.
 // ---------------------------------------------------------------------------
 
-template <int FO, bool MIXED>
+// G: lanes of a particle (Team).
+template <int FO, bool MIXED, int G>
 __global__ void __launch_bounds__(kBlock, 4) k_transport(TransportArgs t, int64_t chunk) {
   const WalkArgs& a = t.mesh;
+  const Team<G> team;
   const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   int64_t cursor = gwarp * chunk;
   const int64_t end = min(t.n, cursor + chunk);
@@ -1126,9 +1212,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_transport(TransportArgs t, int64_
       return true;
     }
     const int32_t nxt = sel4(adj, f);
-    r = add3(r, scl3(ex, u));
+    r = walk_move(team, r, ex, u);
     dist += ex;
-    if (t.tally) atomicAdd(&t.tally[elem], ex);
+    if (t.tally && team.q == 0) atomicAdd(&t.tally[elem], ex);
     if (nxt < -1 || nxt >= a.n_tets) {
       st = RAY_INVALID;  // corrupt adjacency
       return true;
@@ -1144,7 +1230,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_transport(TransportArgs t, int64_
       if (!has) {
         unsigned lt;
         asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-        const int64_t kk = cursor + __popc(need & lt);
+        if (G > 1) lt = (1u << (threadIdx.x & 31 & ~(G - 1))) - 1u;
+        const int64_t kk = cursor + __popc(need & lt) / G;
         if (kk < end) {
           i = kk;
           has = true;
@@ -1160,7 +1247,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_transport(TransportArgs t, int64_
           if (elem >= a.n_tets || !finite3(r) || !finite3(u) || nan_bits(dist)) st = RAY_INVALID;
         }
       }
-      cursor += __popc(need);
+      cursor += __popc(need) / G;
     }
     if (__ballot_sync(0xffffffffu, has) == 0u) break;
     bool done = false;
@@ -1171,10 +1258,11 @@ __global__ void __launch_bounds__(kBlock, 4) k_transport(TransportArgs t, int64_
         done = true;
       }
       if (!done) {
-        cnt.steps++;
+        if (team.q == 0) cnt.steps++;
         double ex;
         const TetRec T = load_rec(a, elem);
-        const int f = next_face<FO, MIXED>(a, T, r, u, sd, sd.safe && in_range3(r), &ex, cnt);
+        const int f = next_face<FO, MIXED, true, G>(a, T, r, u, sd, sd.safe && in_range3(r), &ex, cnt,
+                                                 team);
         // 1 - U of uniform53's U = k 2^-53 is (2^53 - k) 2^-53, exactly
         const unsigned long long U = (1ull << 53) - (splitmix_next(rs) >> 11);
         // Most events leave the tet: an FP32 logarithm with a certified
@@ -1210,9 +1298,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_transport(TransportArgs t, int64_
           const double c = -series_log((double)pu * 1.1102230246251565e-16) * t.mfp;
           if (dlt(c, pex)) {
             // collision inside the tet (:81-85)
-            r = add3(r, scl3(c, u));
+            r = walk_move(team, r, c, u);
             dist += c;
-            if (t.tally) atomicAdd(&t.tally[elem], c);
+            if (t.tally && team.q == 0) atomicAdd(&t.tally[elem], c);
             u = sample_direction(rs);
             sd = step_dir(a, u);
             ++ev;
@@ -1225,6 +1313,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_transport(TransportArgs t, int64_
       }
     }
     if (has && done) {
+      has = false;
+      if (team.q != 0) continue;
       t.elem[i] = elem;
       t.pos[3 * i] = r.x;
       t.pos[3 * i + 1] = r.y;
@@ -1236,22 +1326,21 @@ __global__ void __launch_bounds__(kBlock, 4) k_transport(TransportArgs t, int64_
       t.distance[i] = dist;
       t.events[i] = ev;
       if (t.status) t.status[i] = st;
-      has = false;
       parts++;
     }
   }
   if (t.counters) flush(t.counters, cnt, parts);
 }
 
-template <int FO, bool MIXED>
+template <int FO, bool MIXED, int G = 1>
 cudaError_t launch_transport_t(const TransportArgs& a, cudaStream_t st) {
   static std::atomic<int> cached[kMaxDevices];  // resident blocks per SM, per device
-  auto kern = k_transport<FO, MIXED>;
+  auto kern = k_transport<FO, MIXED, G>;
   int per_sm = 0;
   const cudaError_t e = occupancy_cached(cached, kern, kBlock, 0, per_sm);
   if (e != cudaSuccess) return e;
   int64_t blocks = (int64_t)device_sm_count() * per_sm;
-  const int lanes = lanes_per_warp(a.n, kFp64Warps);
+  const int lanes = std::min(32 / G, lanes_per_warp(a.n, kFp64Warps));
   const int64_t max_blocks = ((a.n + lanes - 1) / lanes + kBlock / 32 - 1) / (kBlock / 32);
   if (blocks > max_blocks) blocks = max_blocks;
   if (blocks < 1) blocks = 1;
@@ -1265,6 +1354,8 @@ cudaError_t launch_transport_t(const TransportArgs& a, cudaStream_t st) {
 
 cudaError_t launch_transport(bool mixed, int face_order, const TransportArgs& a, cudaStream_t st) {
   if (a.n <= 0) return cudaSuccess;
+  if (face_order == 0 && a.n <= (int64_t)device_sm_count() * kTeamWarps * 8)
+    return mixed ? launch_transport_t<0, true, 4>(a, st) : launch_transport_t<0, false, 4>(a, st);
   switch ((face_order == 0 ? 0 : 2) + (mixed ? 1 : 0)) {
     case 0: return launch_transport_t<0, false>(a, st);
     case 1: return launch_transport_t<0, true>(a, st);
