@@ -50,7 +50,7 @@ struct SurfaceRec {
   int32_t rev_tree = -1;
   int32_t bc = 0;  // boundary condition for the particle loop (xdgcu_set_surface_boundary)
   double bump = 0.0;
-  bool int_ok = true;  // every vertex coordinate is in_range_of<60>() (imul64.cuh)
+  bool int_ok = true;  // every vertex coordinate is 0 or 2^-60 .. 2^60 in magnitude
 };
 
 struct TreeHost {
@@ -1570,15 +1570,23 @@ int xdgcu_register_surface(xdgcu_ctx* c, int32_t surface_id, int64_t n_faces, co
     return set_err(XDGCU_ERR_STATE, "register_surface: surface already registered");
   if ((int64_t)c->h_tri_face.size() + n_faces > (int64_t)(1 << 27))
     return set_err(XDGCU_ERR_INVALID_ARG, "register_surface: more than 2^27 triangles");
-  for (int64_t i = 0; i < 9 * n_faces; ++i)
-    if (!(std::fabs(tri_xyz[i]) < 0x1p300))
-      return set_err(XDGCU_ERR_INVALID_ARG,
-                     "register_surface: coordinates must be finite and below 2^300 in magnitude");
+  // one pass: every coordinate sane, and whether all are in closest's range
+  bool sane = true, in60 = true;
+  for (int64_t i = 0; i < 9 * n_faces; ++i) {
+    uint64_t b;
+    std::memcpy(&b, tri_xyz + i, sizeof b);
+    b &= 0x7fffffffffffffffull;
+    sane &= b < (uint64_t)(1023 + 300) << 52;
+    in60 &= (b - ((uint64_t)(1023 - 60) << 52) < (uint64_t)120 << 52) | (b == 0);
+  }
+  if (!sane)
+    return set_err(XDGCU_ERR_INVALID_ARG,
+                   "register_surface: coordinates must be finite and below 2^300 in magnitude");
   SurfaceRec r;
   r.id = surface_id;
   r.first = (int64_t)c->h_tri_face.size();
   r.count = n_faces;
-  for (int64_t i = 0; i < 9 * n_faces; ++i) r.int_ok = r.int_ok && in_range_of<60>(tri_xyz[i]);
+  r.int_ok = in60;
   const int32_t sidx = (int32_t)c->surfs.size();
   c->surf_index[surface_id] = sidx;
   c->surfs.push_back(r);

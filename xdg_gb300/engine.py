@@ -123,7 +123,10 @@ def volume_bounding_box(model, volume):
     lo = np.zeros(3)
     hi = np.zeros(3)
     for s, _ in model.volume_surfaces(volume):
-        x = s.vertices[s.triangles.reshape(-1)]
+        # (each vertex of the surface's triangles once, not once per triangle)
+        used = np.zeros(len(s.vertices), dtype=bool)
+        used[s.triangles.reshape(-1)] = True
+        x = s.vertices[used]
         lo = np.minimum(lo, x.min(0))
         hi = np.maximum(hi, x.max(0))
     return lo, hi
