@@ -9,7 +9,7 @@ from xdg_gb300.engine import FP64, MIXED, XDG, CudaRayTracer
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1, 2, 31, 33, 608, 913, 1825, 2433, 4865, 20000, 24320, 24321]
+SIZES = [1, 2, 31, 33, 608, 913, 1825, 2433, 4865, 20000, 24320, 24321, 29999]
 N = 30000
 
 

@@ -494,8 +494,8 @@ __device__ __forceinline__ void walk_end_state(const WalkArgs& a, int64_t i, d3 
 
 // Where a warp's tracks come from: positions cursor .. end - 1 of the batch,
 // or of the length order.  Without an order, one contiguous chunk.  With one,
-// the warp takes 32 (eight teams: 8) consecutive positions at a time, longest first, from the
-// launch's work counter.  The lanes of a warp then hold tracks of about the
+// the warp takes 32 (of four-lane teams, 8) consecutive positions at a time,
+// longest first, from the launch's work counter.  The lanes of a warp then hold tracks of about the
 // same length and end together, so the FP64 unit, which takes as long for one
 // lane as for 32, sees full warps (dealt one by one, every warp held one of
 // the longest tracks and stepped on for it alone), and the warps end together
@@ -504,29 +504,38 @@ __device__ __forceinline__ void walk_end_state(const WalkArgs& a, int64_t i, d3 
 template <int G = 1>
 struct WarpTracks {
   static constexpr int kTake = 32 / G;  // tracks a warp holds
-  int64_t cursor, end;
+  int64_t cursor, end, last;  // `last`: the end of its part of the order
+  unsigned long long* work;   // that part's work counter, from its first position `first`
+  int64_t first;
+  bool open;                  // the order may hold more
   __device__ __forceinline__ WarpTracks(const WalkArgs& a, int64_t gwarp, int64_t chunk) {
     cursor = a.order ? 0 : gwarp * chunk;
     end = a.order ? 0 : min(a.n, cursor + chunk);
+    part(a, 0, a.n, 0);
   }
-  __device__ __forceinline__ bool more(const WalkArgs& a) const {
-    return cursor < end || (a.order && end <= a.n);
+  // positions first_ .. last_ - 1 of the order, by work counter k
+  __device__ __forceinline__ void part(const WalkArgs& a, int64_t first_, int64_t last_, int k) {
+    first = first_;
+    last = last_;
+    work = a.order ? a.work + k : nullptr;
+    open = a.order != nullptr;
   }
+  __device__ __forceinline__ bool more() const { return cursor < end || open; }
   // the track of the `rank`-th of `want` lanes, or -1 (warp-uniform but for
   // rank; all lanes of the warp call it)
   __device__ __forceinline__ int64_t take(const WalkArgs& a, int rank, int want) {
-    if (a.order && cursor >= end && end <= a.n) {
+    if (cursor >= end && open) {
       unsigned long long base = 0ull;
-      if ((threadIdx.x & 31) == 0) base = atomicAdd(a.work, (unsigned long long)kTake);
+      if ((threadIdx.x & 31) == 0) base = atomicAdd(work, (unsigned long long)kTake);
       base = __shfl_sync(0xffffffffu, base, 0);
-      cursor = (int64_t)base;
-      // (end stays past n once the order is used up, and no more is taken)
-      end = cursor < a.n ? min(a.n, cursor + kTake) : a.n + 1;
-      if (cursor >= a.n) cursor = end;
+      cursor = first + (int64_t)base;
+      end = min(last, cursor + kTake);
+      open = end > cursor;
+      if (!open) cursor = end = 0;
     }
     const int64_t pos = cursor + rank;
     cursor = min(end, cursor + want);
-    if (pos >= end || pos >= a.n) return -1;
+    if (pos >= end) return -1;
     if (!a.order) return pos;
     const int64_t i = __ldg(&a.order[pos]);
     return i >= 0 && i < a.n ? i : -1;  // (an entry out of range names no track)
@@ -538,15 +547,11 @@ struct WarpTracks {
 // lengths are exponentially distributed, so one-track-per-lane would leave
 // most lanes idle behind the longest track of the warp).
 // SUM: the running length sum is wanted (WalkArgs::sum_out).  INT: products on
-// the integer pipes (next_face).
-// G: lanes of a track (Team).
+// the integer pipes (next_face).  G: lanes of a track (Team).
 template <int FO, bool MIXED, bool SUM, bool INT, int G>
-__global__ void __launch_bounds__(kBlock, 4) k_walk(WalkArgs a, int64_t chunk) {
+__device__ __forceinline__ void walk_tracks(const WalkArgs& a, WarpTracks<G> list, StepCnt& cnt,
+                                            unsigned long long& tracks) {
   const Team<G> team;
-  const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  WarpTracks<G> list(a, gwarp, chunk);
-  StepCnt cnt = {0, 0};
-  unsigned long long tracks = 0;
   bool has = false;
   int64_t i = 0;
   d3 r = mk3(0, 0, 0), u = mk3(0, 0, 0);
@@ -599,7 +604,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(WalkArgs a, int64_t chunk) {
       }
     }
     if (__ballot_sync(0xffffffffu, has) == 0u) {
-      if (list.more(a)) continue;
+      if (list.more()) continue;
       break;
     }
     if (has) {
@@ -652,8 +657,36 @@ __global__ void __launch_bounds__(kBlock, 4) k_walk(WalkArgs a, int64_t chunk) {
       }
     }
   }
+}
+
+template <int FO, bool MIXED, bool SUM, bool INT, int G>
+__global__ void __launch_bounds__(kBlock, 4) k_walk(WalkArgs a, int64_t chunk) {
+  const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  StepCnt cnt = {0, 0};
+  unsigned long long tracks = 0;
+  walk_tracks<FO, MIXED, SUM, INT, G>(a, WarpTracks<G>(a, gwarp, chunk), cnt, tracks);
   if (a.counters) flush(a.counters, cnt, tracks);
 }
+
+// A walk in length order that lasts as long as its longest tracks: the first
+// `team_blocks` blocks walk the first n_team of the order four lanes to a
+// track (Team), the others the rest, and then they help.
+template <int FO, bool MIXED>
+__global__ void __launch_bounds__(kBlock, 4) k_walk_mix(WalkArgs a, int64_t n_team,
+                                                        unsigned team_blocks) {
+  StepCnt cnt = {0, 0};
+  unsigned long long tracks = 0;
+  if (blockIdx.x < team_blocks) {
+    WarpTracks<4> list(a, 0, 0);
+    list.part(a, 0, n_team, 0);
+    walk_tracks<FO, MIXED, false, MIXED, 4>(a, list, cnt, tracks);
+  }
+  WarpTracks<1> list(a, 0, 0);
+  list.part(a, n_team, a.n, 1);
+  walk_tracks<FO, MIXED, false, true, 1>(a, list, cnt, tracks);
+  if (a.counters) flush(a.counters, cnt, tracks);
+}
+
 
 template <int FO, bool MIXED>
 __global__ void __launch_bounds__(kBlock) k_next(WalkArgs a) {
@@ -840,7 +873,7 @@ __global__ void __launch_bounds__(kBlock) k_walk_q(WalkArgs a, int64_t chunk) {
       }
     }
     if (__ballot_sync(0xffffffffu, has) == 0u) {
-      if (list.more(a)) continue;
+      if (list.more()) continue;
       break;
     }
 
@@ -1125,6 +1158,33 @@ cudaError_t launch_walk_s(const WalkArgs& a, cudaStream_t st) {
 // 3.44 / 3.30 / 3.32, 60,000 4.07 / 4.07 / 4.24.
 constexpr int kTeamWarps = 20;
 
+// k_walk_mix: one in kMixPart of the tracks, the longest, in teams, on at most
+// a third of the resident blocks, for batches of up to kMixWarps * 32 tracks
+// per SM (107,008).  Located and walked, without / with, ms: 28,000 tracks
+// 1.91 / 1.54 mixed, 2.57 / 2.06 all-FP64; 50,000 2.16 / 1.71 and 3.46 / 2.30;
+// 100,000 2.42 / 2.07 and 3.95 / 2.81 (an eighth in teams 2.26 and 3.18, a quarter
+// 2.65 and 3.58); 200,000, an eighth, 2.75 / 3.59 and 4.44 / 4.87.  Not for the
+// global loop's walks, whose order is by the track's length and not the walk's:
+// 50,000 tracks 4.00 / 4.17.
+constexpr int kMixPart = 14, kMixWarps = 22;
+
+template <int FO, bool MIXED>
+cudaError_t launch_walk_mix(const WalkArgs& a, cudaStream_t st) {
+  static std::atomic<int> cached[kMaxDevices];
+  auto kern = k_walk_mix<FO, MIXED>;
+  int per_sm = 0;
+  cudaError_t e = occupancy_cached(cached, kern, kBlock, 0, per_sm);
+  if (e == cudaSuccess) e = cudaMemsetAsync(a.work, 0, 2 * sizeof(*a.work), st);
+  if (e != cudaSuccess) return e;
+  const int64_t resident = (int64_t)device_sm_count() * per_sm;
+  const int64_t n_team = a.n / kMixPart / 8 * 8;
+  const int64_t team_blocks = std::min((n_team + 31) / 32, std::max<int64_t>(1, resident / 3));
+  const int64_t rest = std::min((a.n - n_team + kBlock - 1) / kBlock,
+                                std::max<int64_t>(1, resident - team_blocks));
+  kern<<<(unsigned)(team_blocks + rest), kBlock, 0, st>>>(a, n_team, (unsigned)team_blocks);
+  return cudaGetLastError();
+}
+
 template <int FO, bool MIXED, bool QUEUE>
 cudaError_t launch_walk_t(const WalkArgs& a, cudaStream_t st) {
   // With at most about one warp a scheduler a step is a chain, and in the
@@ -1132,10 +1192,13 @@ cudaError_t launch_walk_t(const WalkArgs& a, cudaStream_t st) {
   // (1,000 tracks located and walked 2.11 ms with the integer products, 1.84
   // without; 20,000 3.25 and 2.49; 60,000 3.71 and 4.27)
   const int64_t team_max = (int64_t)device_sm_count() * kTeamWarps * 8;
-  if constexpr (FO == 0 && !QUEUE)
+  if constexpr (FO == 0 && !QUEUE) {
     if (a.n <= team_max)
       return a.sum_out ? launch_walk_s<FO, MIXED, false, true, MIXED, 4>(a, st)
                        : launch_walk_s<FO, MIXED, false, false, MIXED, 4>(a, st);
+    if (a.order && !a.sum_out && a.n <= (int64_t)device_sm_count() * kMixWarps * 32)
+      return launch_walk_mix<FO, MIXED>(a, st);
+  }
   if (!MIXED && a.n <= (int64_t)device_sm_count() * kFp64Warps * 32)
     return a.sum_out ? launch_walk_s<FO, MIXED, QUEUE, true, MIXED>(a, st)
                      : launch_walk_s<FO, MIXED, QUEUE, false, MIXED>(a, st);

@@ -56,7 +56,7 @@ struct WalkArgs {
   // mixed walk: 1 = per-warp FP64 queue (k_walk_q), 0 = per-lane escalation
   int32_t walk_queue;
   // optional: track indices by decreasing length; the warps then take them 32
-  // at a time, longest first, from the work counter (zero at launch)
+  // at a time, longest first, from the work counters (two, zeroed by the launch)
   const int32_t* order;
   unsigned long long* work;
   int32_t flush_wait;  // queue: lanes waiting that force a partial FP64 round
