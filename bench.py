@@ -95,13 +95,15 @@ NOALLOC_MAX_TRACKS = 4_194_304
 # a division counted as one:
 #   per step: cross(u, r) 9 (plucker.h:75), r += len * u and distance -= len 7;
 #   per face tested exactly from the edge table: 3 coordinates x 11
-#   (dot(u, e x lo) + dot(u x r, e)) + 14 for the hit distance (sum, 1/sum,
-#   3 weights, the hit point component, its difference and quotient, u + v);
-#   the all-FP64 path computes each coordinate from the vertices (23: edge,
-#   cross, two dots, sum), 4 faces per step, one of which reaches the distance.
+#   (dot(u, e x lo) + dot(u x r, e)) + the hit distance (sum, 1/sum,
+#   3 weights, the hit point component, its difference and quotient: 13);
+#   the all-FP64 path evaluates the tet's six edge coordinates, and one face's
+#   distance.
+# The products among them (30 mixed, 48 all-FP64) run on the integer pipes; the
+# fraction is of all operations against the FP64 unit's rate.
 WALK_FP64_OPS_STEP = 16
-WALK_FP64_OPS_FACE = 47
-WALK_FP64_OPS_FP64_PATH = 16 + 4 * 69 + 14
+WALK_FP64_OPS_FACE = 46
+WALK_FP64_OPS_FP64_PATH = 16 + 6 * 11 + 13
 # bytes per segment (conn 16 + adjacency 16 + 4 FP32 vertices 48 + output 12)
 WALK_BYTES_SEG_MIXED = 92
 
