@@ -279,3 +279,34 @@ def test_simulate_particles_facade(cuda):
     assert abs(sum(res["tally"].values()) - res["distance"].sum()) < 1e-9 * res["distance"].sum()
     with pytest.raises(Exception):
         x.rti.set_surface_boundary({77: BC_VACUUM})
+
+
+def _state_before(z):
+    """The SplitMix64 state whose next output is z."""
+    mask = (1 << 64) - 1
+    z ^= (z >> 31) ^ (z >> 62)
+    z = z * pow(0x94D049BB133111EB, -1, 1 << 64) & mask
+    z ^= (z >> 27) ^ (z >> 54)
+    z = z * pow(0xBF58476D1CE4E5B9, -1, 1 << 64) & mask
+    z ^= (z >> 30) ^ (z >> 60)
+    return (z - 0x9E3779B97F4A7C15) & mask
+
+
+@pytest.mark.parametrize("prec", [FP64, MIXED])
+def test_streams_at_the_ends_of_the_uniform(cube, oracle, prec):
+    """Streams whose first or second draw k (U = k 2^-53) is at the ends of its
+    range, around the powers of two and at the middle, where 2 U - 1 is 0."""
+    m, x, elem, p, u = cube
+    ks = sorted({min(max(b + d, 0), 2**53 - 1) for b in [0, 2**53, *(2**i for i in range(1, 53))]
+                 for d in (-1, 0, 1)} | {2**53 - 2**i for i in range(1, 53)})
+    golden = 0x9E3779B97F4A7C15
+    seeds = [_state_before(k << 11) for k in ks]
+    seeds += [(s - golden) % 2**64 for s in seeds]
+    seeds = np.array(seeds, dtype=np.uint64)
+    n = len(seeds)
+    o = _oracle_walker(oracle, m).transport(elem[:n], p[:n], u[:n], seeds, 0.5, 40)
+    e, r, d, s = elem[:n].copy(), p[:n].copy(), u[:n].copy(), seeds.copy()
+    dist, ev = np.zeros(n), np.zeros(n, dtype=np.int32)
+    st = x.rti.transport_elements(e, r, d, s, 0.5, 40, dist, ev, None, precision=prec)
+    for k, (name, a) in enumerate(zip(NAMES, [e, r, d, s, dist, ev, st])):
+        assert_same(a, o[k], name)

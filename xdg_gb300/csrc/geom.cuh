@@ -417,7 +417,7 @@ __device__ __forceinline__ float f32_trunc(double x) {
 // used for the culling distance; +inf for DBL_MAX or inf.
 __device__ __forceinline__ float f32_up(double x) {
   const float t = f32_trunc(x);
-  if (!(x > 0.0)) return t;
+  if (!gt0(x)) return t;
   const unsigned tb = __float_as_uint(t);
   return (tb >= 0x7f800000u) ? __uint_as_float(0x7f800000u) : __uint_as_float(tb + 1u);
 }

@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(kTBlock, MINB) k_trace(SurfArgs a, int64_t chu
         d3 o = ray_o(tx), d = ray_d(tx);
         bool alive = false;
         if (status == RAY_OK && tid > 0) {
-          if (bhas && bt == 0.0) {
+          if (bhas && is0(bt)) {
             status = RAY_STUCK;  // :36-40
           } else if (!bhas) {
             status = RAY_LOST;   // :41-45
@@ -371,30 +371,29 @@ __global__ void __launch_bounds__(kTBlock, MINB) k_trace(SurfArgs a, int64_t chu
             // particle may collide: an FP32 logarithm with a certified margin
             // (|c32 - c| <= 6.1e-8 mfp + 3.7e-7 c; margin 1.1e-6 (c32 + mfp))
             // first tests c >= hit distance.
-            const double U = uniform53(rs);
+            const unsigned long long R = (1ull << 53) - uniform_bits(rs);  // (1 - U) 2^53
             bool cross = false;
             if (a.mfp < 1e30) {
               const float mfp32 = (float)a.mfp;
-              const float c32 = -logf(__double2float_rn(1.0 - U)) * mfp32;
-              cross = dlt(bt, (double)(c32 - 1.1e-6f * (c32 + mfp32)));
+              const float c32 = -logf(__ull2float_rn(R) * 1.1102230246251565e-16f) * mfp32;
+              cross = f32_up(bt) < c32 - 1.1e-6f * (c32 + mfp32);
             }
             double c = 0.0;
-            if (!cross) c = -series_log(1.0 - U) * a.mfp;  // sample_collision's value
+            if (!cross) c = -series_log(unit_scaled(R, -53)) * a.mfp;  // the collision distance
             alive = true;
-            if (!cross && dlt(c, bt)) {
-              // advance + collide (:66-70, :57-64)
-              o = add3(o, scl3(c, d));
-              pdist += c;
-              if (a.p_tally) atomicAdd(&a.p_tally[tid], c);
-              ++pev;
+            // advance (:66-70, :71-75)
+            const bool collide = !cross && dlt(c, bt);
+            const double len = collide ? c : bt;
+            o = add3(o, scl3(len, d));
+            pdist += len;
+            if (a.p_tally) atomicAdd(&a.p_tally[tid], len);
+            ++pev;
+            if (collide) {
+              // collide (:57-64)
               d = sample_direction(rs);
               hc = 0;
             } else {
-              // advance to the surface + cross_surface (:71-75, :78-118)
-              o = add3(o, scl3(bt, d));
-              pdist += bt;
-              if (a.p_tally) atomicAdd(&a.p_tally[tid], bt);
-              ++pev;
+              // cross_surface (:78-118)
               const int32_t sidx = __ldg(&a.tri_surf[btri]);
               const int32_t bc = __ldg(&a.surf_bc[sidx]);
               if (bc == BC_REFLECTING) {

@@ -1326,8 +1326,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_transport(TransportArgs t, int64_
         const TetRec T = load_rec(a, elem);
         const int f = next_face<FO, MIXED, true, G>(a, T, r, u, sd, sd.safe && in_range3(r), &ex, cnt,
                                                  team);
-        // 1 - U of uniform53's U = k 2^-53 is (2^53 - k) 2^-53, exactly
-        const unsigned long long U = (1ull << 53) - (splitmix_next(rs) >> 11);
+        // 1 - U of U = k 2^-53 is (2^53 - k) 2^-53, exactly
+        const unsigned long long U = (1ull << 53) - uniform_bits(rs);
         // Most events leave the tet: an FP32 logarithm with a certified
         // margin decides c >= exit without the FP64 series.  |c32 - c| <=
         // 6.1e-8 mfp + 3.7e-7 c (rounding 1 - U to FP32, logf within 2 ulp,
@@ -1336,7 +1336,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_transport(TransportArgs t, int64_
         if (quick) {
           const float c32 = -logf(__ull2float_rn(U) * 1.1102230246251565e-16f) * mfp32;
           const float lo = c32 - 1.1e-6f * (c32 + mfp32);
-          leaves = dlt(ex, (double)lo);  // c >= lo > exit
+          leaves = f32_up(ex) < lo;  // c >= lo > exit
         }
         if (leaves) {
           done = exit_step(ex, f, T.adj);
@@ -1357,8 +1357,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_transport(TransportArgs t, int64_
       if (__popc(pm) >= t.event_wait || run == 0u) {
         if (has && pend) {
           pend = false;
-          // sample_collision's value
-          const double c = -series_log((double)pu * 1.1102230246251565e-16) * t.mfp;
+          // the collision distance
+          const double c = -series_log(unit_scaled(pu, -53)) * t.mfp;
           if (dlt(c, pex)) {
             // collision inside the tet (:81-85)
             r = walk_move(team, r, c, u);
