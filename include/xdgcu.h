@@ -481,14 +481,17 @@ int xdgcu_get_counters(xdgcu_ctx* ctx, int64_t counters[8]);
  *                      one contiguous slice fixed at launch
  *   "particle_event_wait"  particle loop of xdgcu_transport_surfaces: lanes
  *                      whose flights have ended that a warp gathers before it
- *                      runs their events together (1..32, default 20: 1e6
- *                      particles of the nested spheres 76.4 / 76.2 / 78.9 ms
+ *                      runs their events together, unless at most one lane of
+ *                      the warp still traverses (1..32, default 20: 1e6
+ *                      particles of the nested spheres 74.0 / 70.4 / 85.7 ms
  *                      with 16 / 20 / 24)
  *   "transport_event_wait" particle loop of xdgcu_transport_elements: lanes
  *                      whose events need the FP64 sample (collisions,
  *                      uncertain exits) that a warp gathers before it runs
  *                      them together, in batches that give every lane a
- *                      particle (1..32, default 4; smaller batches never wait)
+ *                      particle (1..32, default 4; smaller batches never wait,
+ *                      mixed ones of eight particles a lane wait for at
+ *                      least 8)
  *   "trace_sort_min"   batches of at least this many rays (default 0 = never)
  *                      are traversed in a coherent order: sorted on the device
  *                      by tree, direction octant and the Morton code of the

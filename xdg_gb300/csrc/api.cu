@@ -3034,9 +3034,11 @@ int xdgcu_transport_surfaces(xdgcu_ctx* c, int64_t n, int32_t* tree, double* pos
   a.event_wait = c->particle_event_wait;
   const bool mixed = precision == XDGCU_MIXED;
   // Where every lane has a particle, the others' work covers a longer wait for
-  // fuller drains (1e6 particles of the nested spheres, event_wait 20: 79.9 ms
-  // flushing at 4 waiting lanes, 76.2 at 8; 20,000 particles 17.1 and 17.4)
-  if (mixed && n >= (int64_t)device_sm_count() * 16 * 32) a.flush_wait = std::max(a.flush_wait, 8);
+  // fuller drains.  With event_wait 20 a wait for 12 lanes leaves two lanes
+  // searching at the least, and the pair is a sharp best (1e6 particles of
+  // the nested spheres, ms with 8 / 12 / 16 lanes: 73.9 / 70.4 / 72.2, 3e6 191 /
+  // 183 / 185, 200,000 29.2 / 28.2 / 28.2; event_wait 24 with 12: 85.7)
+  if (mixed && n >= (int64_t)device_sm_count() * 16 * 32) a.flush_wait = std::max(a.flush_wait, 12);
   cudaStream_t st = (cudaStream_t)stream;
   auto bind = [&](char* const* p) {
     a.p_tree = (int32_t*)p[0];
@@ -3137,8 +3139,13 @@ int xdgcu_transport_elements(xdgcu_ctx* c, int64_t n, int32_t* elem_index, doubl
   // particle; before that the lanes that wait are what the launch waits for
   // (ms with 1 / 2 / 4 lanes, mixed: 20,000 particles 11.5 / 12.1 / 12.2, 200,000
   // 25.7 / 23.8 / 23.6; FP64: 14.8 / 15.6 / 15.8 and 34.0 / 32.2 / 32.6)
-  t.event_wait = n >= (int64_t)device_sm_count() * 16 * 32 ? c->transport_event_wait : 1;
+  // and, mixed, fuller ones where a lane runs many particles (ms with 4 / 8 lanes:
+  // 600,000 particles 38.8 / 38.6, 1e6 53.6 / 51.7, 3e6 128.8 / 118.0; FP64
+  // 600,000 52.4 / 53.6).
   const bool mixed = precision == XDGCU_MIXED;
+  const int64_t full = (int64_t)device_sm_count() * 16 * 32;  // a particle for every lane
+  t.event_wait = n >= full ? c->transport_event_wait : 1;
+  if (mixed && n >= 8 * full) t.event_wait = std::max(t.event_wait, 8);
   cudaStream_t st = (cudaStream_t)stream;
   if (kind == 1) {
     t.elem = elem_index;
