@@ -363,7 +363,7 @@ __device__ __forceinline__ int next_face(const WalkArgs& a, const TetRec& T, d3 
         if (!out && !zero) escm |= 1u << f;
       }
     }
-    cnt.esc += 4;
+    if (team.q == 0) cnt.esc += 4;  // (a team's lanes share one step)
   } else {
     float4 P[4];
 #pragma unroll
@@ -420,7 +420,7 @@ __device__ __forceinline__ int next_face(const WalkArgs& a, const TetRec& T, d3 
   while (escm) {
     const int f = __ffs(escm) - 1;
     escm &= escm - 1u;
-    if (MIXED) cnt.esc++;
+    if (MIXED && team.q == 0) cnt.esc++;
     const int l0 = face_local<FO>(a, f, 0), l1 = face_local<FO>(a, f, 1),
               l2 = face_local<FO>(a, f, 2);
     const int32_t i0 = sel4(ci, l0), i1 = sel4(ci, l1), i2 = sel4(ci, l2);
