@@ -215,7 +215,8 @@ __device__ __noinline__ double face_exit_xyz(const double* xyz, int32_t i0, int3
 
 // FP32 value nearest to x (to even), by integer operations: a conversion
 // instruction holds the FP64 unit for 33 ns a warp.  Magnitudes below FLT_MIN
-// give 0 (an error below 2^-126, far inside the filter's absolute term).
+// give 0 (an error below 2^-126: of a position far inside the filter's
+// absolute term, of a direction see step_dir).
 __device__ __forceinline__ float f32_near(double x) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const unsigned long long q = b + 0x0fffffffull + ((b >> 29) & 1ull);
@@ -229,7 +230,7 @@ __device__ __forceinline__ float f32_near(double x) {
 
 // What a step needs of the track's direction, set when it changes.
 struct StepDir {
-  float x, y, z;  // FP32, nearest
+  float x, y, z;  // FP32, nearest (x is NaN where FP32 may not decide)
   int axis;       // plucker_axis
   bool safe;      // the mesh and the direction are in range (imul64.cuh)
 };
@@ -239,6 +240,10 @@ __device__ __forceinline__ StepDir step_dir(const WalkArgs& a, d3 u) {
   s.x = f32_near(u.x);
   s.y = f32_near(u.y);
   s.z = f32_near(u.z);
+  // The filter's bound has a term u D W^2 for the direction's rounding, which
+  // covers a component flushed to zero (2^-126 W^2) only for a longer D; with
+  // NaN no FP32 coordinate is above the bound and every face is tested.
+  if (!(fmaxf(fabsf(s.x), fmaxf(fabsf(s.y), fabsf(s.z))) >= 0x1p-100f)) s.x = NAN;
   s.axis = plucker_axis(u);
   s.safe = a.edge && a.int_ok && in_range3(u);
   return s;
