@@ -473,12 +473,16 @@ int xdgcu_get_counters(xdgcu_ctx* ctx, int64_t counters[8]);
  *                      XDGCU_RAY_STACK_OVERFLOW
  *   "trace_grab"       > 0 (a multiple of 32): warps take this many rays at a
  *                      time from a device work queue, which balances batches of
- *                      very uneven per-ray cost; 0 (default): by the batch --
- *                      mixed ray_fire, point_in_volume and occluded of at least
- *                      2e6 rays take 64 at a time, find_volume and
- *                      point_in_volumes of at least 5e5 points 32, and other
- *                      launches (and those captured in a graph) give each warp
- *                      one contiguous slice fixed at launch
+ *                      very uneven per-ray cost; 0 (default): as trace_queue
+ *                      says
+ *   "trace_queue"      where trace_grab is 0: 1 (default) by the batch -- mixed
+ *                      ray_fire, point_in_volume and occluded of at least 2e6
+ *                      rays take 64 at a time, find_volume and
+ *                      point_in_volumes of at least 5e5 points 32 (the queue's
+ *                      cursor is temporary memory; without any, and in
+ *                      launches captured in a graph, slices), and other
+ *                      launches give each warp one contiguous slice fixed at
+ *                      launch; 0: slices always
  *   "particle_event_wait"  particle loop of xdgcu_transport_surfaces: lanes
  *                      whose flights have ended that a warp gathers before it
  *                      runs their events together, unless at most one lane of
@@ -577,7 +581,11 @@ int xdgcu_get_counters(xdgcu_ctx* ctx, int64_t counters[8]);
  *                      XDGCU_SCRATCH_POOL=0 in the environment when the
  *                      context is created, the device's default pool serves
  *                      instead (for tools that save and restore device
- *                      memory, such as a profiler's kernel replay).  Read-only
+ *                      memory, such as a profiler's kernel replay).  With
+ *                      XDGCU_SCRATCH_LIMIT=bytes there a call's temporary
+ *                      memory past that many bytes is refused as on a device
+ *                      that has no more (for testing what the calls do then).
+ *                      Read-only
  *                      "scratch_bytes_reserved" is what the pool holds and
  *                      "scratch_bytes_high" the most it has lent at once
  *                      (set it to 0 to restart the count)

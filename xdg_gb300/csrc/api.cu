@@ -556,7 +556,8 @@ struct xdgcu_ctx {
   int32_t trace_node_iters_direct = 6;  // mixed launches reading their rays in place from host memory
   int32_t trace_flush_wait = 4;
   int32_t trace_stack = 40;      // shared-memory stack entries per lane
-  int32_t trace_grab = 0;        // 0: one contiguous chunk per warp; > 0: device work queue
+  int32_t trace_grab = 0;        // > 0: rays a warp takes from the device work queue; 0: see trace_queue
+  int32_t trace_queue = 1;       // trace_grab 0: 1 by the batch (queue_grab_for), 0 one contiguous chunk per warp
   int64_t trace_sort_min = 0;    // batches of at least this many rays run in coherent order (0 = never)
   int32_t surf_width8 = 0;            // some surface tree has 8-wide nodes
   int32_t surf_stack_bound = 0;       // largest (width - 1) * depth of the surface trees
@@ -610,12 +611,16 @@ struct xdgcu_ctx {
   // global track loop on 1e6 tracks: 36.7 -> 33.0 ms); null: the default pool
   cudaMemPool_t pool = nullptr;
   int64_t keep_bytes = int64_t(8) << 30;
+  // most scratch bytes of a call (0: what the device has); stands in for a
+  // device without free memory in the tests of the paths for that
+  size_t scratch_limit = 0;
 };
 
 namespace {
 
 // Stream-ordered scratch of a call, from the context's pool.
 cudaError_t scratch_alloc(const xdgcu_ctx* c, void** p, size_t bytes, cudaStream_t s) {
+  if (c->scratch_limit && bytes > c->scratch_limit) return cudaErrorMemoryAllocation;
   return c->pool ? cudaMallocFromPoolAsync(p, bytes, c->pool, s) : cudaMallocAsync(p, bytes, s);
 }
 
@@ -1155,10 +1160,11 @@ int with_length_order(xdgcu_ctx* c, WalkArgs& a, cudaStream_t s, Body body) {
 
 // Stream-ordered scratch of one call, freed on every return path.
 struct CallScratch {
+  const xdgcu_ctx* c;
   cudaStream_t st;
-  cudaMemPool_t pool;
   std::vector<void*> ptrs;
-  CallScratch(cudaStream_t s, cudaMemPool_t p) : st(s), pool(p) {}
+  size_t held = 0;
+  CallScratch(const xdgcu_ctx* ctx, cudaStream_t s) : c(ctx), st(s) {}
   ~CallScratch() {
     for (void* p : ptrs) cudaFreeAsync(p, st);
   }
@@ -1167,10 +1173,11 @@ struct CallScratch {
     *out = nullptr;
     void* p = nullptr;
     const size_t bytes = sizeof(T) * (size_t)std::max<int64_t>(1, count);
-    const cudaError_t e =
-        pool ? cudaMallocFromPoolAsync(&p, bytes, pool, st) : cudaMallocAsync(&p, bytes, st);
+    if (c->scratch_limit && held + bytes > c->scratch_limit) return cudaErrorMemoryAllocation;
+    const cudaError_t e = scratch_alloc(c, &p, bytes, st);
     if (e != cudaSuccess) return e;
     ptrs.push_back(p);
+    held += bytes;
     *out = static_cast<T*>(p);
     return cudaSuccess;
   }
@@ -1321,7 +1328,7 @@ int walk_packed_rounds(xdgcu_ctx* c, bool mixed, const WalkArgs& a, cudaStream_t
                        bool* no_memory) {
   *no_memory = false;
   const int64_t n = a.n;
-  CallScratch S(st, c->pool);
+  CallScratch S(c, st);
   bool ok = true;
   auto get = [&](auto** p, int64_t count) {
     if (ok && S.get(p, count) != cudaSuccess) {
@@ -1400,10 +1407,6 @@ int walk_packed_rounds(xdgcu_ctx* c, bool mixed, const WalkArgs& a, cudaStream_t
   return XDGCU_OK;
 }
 
-// Enqueues one traversal launch with the context's work distribution: when
-// the device work queue is on (trace_grab > 0) a zeroed cursor, and when the
-// batch is large enough (trace_sort_min) a coherent ray order, both in one
-// stream-ordered scratch allocation freed after the launch.
 // Stack entries of a traversal launch: the requested depth, raised to the
 // surface trees' bound (width - 1) * depth -- which no traversal can exceed --
 // as far as the 64-entry maximum allows.
@@ -1412,8 +1415,8 @@ int32_t trace_stack_for(const xdgcu_ctx* c) {
   return std::max(c->trace_stack, need);
 }
 
-// Rays a warp takes at a time from the device work queue where trace_grab
-// leaves the choice open (0), or 0 for fixed slices.  The queue evens out the
+// Rays a warp takes at a time from the device work queue where trace_grab and
+// trace_queue leave the choice open (0 and 1), or 0 for fixed slices.  The queue evens out the
 // ends of large batches; its counter has to be allocated and zeroed, and with
 // few rays a warp the last chunks are uneven work again.  Nested spheres, ms
 // with slices / 32 / 64 rays: ray_fire of 1e6 0.686 / 0.677 / 0.689, 2e6 1.265 /
@@ -1432,13 +1435,20 @@ int32_t queue_grab_for(int mode, bool mixed, int64_t n, cudaStream_t s) {
   return cap != cudaStreamCaptureStatusNone ? 0 : (restarts ? 32 : 64);
 }
 
+// Enqueues one traversal launch with the context's work distribution: where
+// the device work queue serves it (trace_grab, queue_grab_for) a zeroed cursor,
+// and when the batch is large enough (trace_sort_min) a coherent ray order,
+// both in one stream-ordered scratch allocation freed after the launch.  A
+// queue that was only the batch's choice gives way to fixed slices where that
+// allocation fails.
 cudaError_t launch_trace(xdgcu_ctx* c, int mode, bool mixed, SurfArgs a, double extent,
                          cudaStream_t s, int32_t min_grab = 0) {
   if (a.n <= 0) return cudaSuccess;
   const bool sort = c->trace_sort_min > 0 && a.n >= c->trace_sort_min && a.n < ((int64_t)1 << 31) &&
                     extent > 0.0;
   a.grab = std::max(c->trace_grab, min_grab);
-  if (a.grab == 0) a.grab = queue_grab_for(mode, mixed, a.n, s);
+  const bool by_batch = a.grab == 0 && c->trace_queue;
+  if (by_batch) a.grab = queue_grab_for(mode, mixed, a.n, s);
   a.work = nullptr;
   a.order = nullptr;
   if (a.grab == 0 && !sort) return launch_surface_query(mode, mixed, a, s);
@@ -1446,6 +1456,11 @@ cudaError_t launch_trace(xdgcu_ctx* c, int mode, bool mixed, SurfArgs a, double 
   const size_t scr = sort ? ray_order_scratch_bytes(a.n) : 0;
   char* buf = nullptr;
   cudaError_t e = scratch_alloc(c, (void**)&buf, 256 + ord_bytes + scr, s);
+  if (e != cudaSuccess && by_batch && !sort) {
+    cudaGetLastError();  // the failed allocation is not a pending launch error
+    a.grab = 0;
+    return launch_surface_query(mode, mixed, a, s);
+  }
   if (e != cudaSuccess) return e;
   if (a.grab > 0) {
     a.work = (unsigned long long*)buf;
@@ -1546,6 +1561,8 @@ int xdgcu_create(xdgcu_ctx** out, int device) {
     cudaGetLastError();
     c->pool = nullptr;
   }
+  if (const char* limit = std::getenv("XDGCU_SCRATCH_LIMIT"))
+    c->scratch_limit = (size_t)std::strtoull(limit, nullptr, 10);
   *out = c;
   return XDGCU_OK;
 }
@@ -1876,6 +1893,9 @@ int xdgcu_set_tuning(xdgcu_ctx* c, const char* key, int64_t value) {
     if (value < 0 || value > (1 << 20) || value % 32 != 0)
       return set_err(XDGCU_ERR_INVALID_ARG, "trace_grab must be 0 or a multiple of 32 up to 2^20");
     c->trace_grab = (int32_t)value;
+  } else if (k == "trace_queue") {
+    if (value < 0 || value > 1) return set_err(XDGCU_ERR_INVALID_ARG, "trace_queue must be 0 or 1");
+    c->trace_queue = (int32_t)value;
   } else if (k == "transport_event_wait") {
     if (value < 1 || value > 32)
       return set_err(XDGCU_ERR_INVALID_ARG, "transport_event_wait must be 1..32");
@@ -1993,6 +2013,7 @@ int xdgcu_get_tuning(const xdgcu_ctx* c, const char* key, int64_t* value) {
   else if (k == "trace_flush_wait") *value = c->trace_flush_wait;
   else if (k == "trace_stack") *value = c->trace_stack;
   else if (k == "trace_grab") *value = c->trace_grab;
+  else if (k == "trace_queue") *value = c->trace_queue;
   else if (k == "trace_sort_min") *value = c->trace_sort_min;
   else if (k == "particle_event_wait") *value = c->particle_event_wait;
   else if (k == "transport_event_wait") *value = c->transport_event_wait;
@@ -2352,7 +2373,7 @@ static int point_query(xdgcu_ctx* c, bool closest, int32_t tree, const int32_t* 
     a.status = status;
     int rc = begin_query(c, st, &a.counters);
     if (rc) return rc;
-    CallScratch S(st, c->pool);
+    CallScratch S(c, st);
     API_CUDA(defer_scratch(S), "closest scratch");
     API_CUDA(launch(), "query launch");
     return XDGCU_OK;
@@ -2361,7 +2382,7 @@ static int point_query(xdgcu_ctx* c, bool closest, int32_t tree, const int32_t* 
   if (!s) return set_err(XDGCU_ERR_CUDA, "staging stream creation failed");
   // (the chunks' launches alternate between the slot's streams; the second
   // waits for the first before its first launch)
-  CallScratch S(s->stream, c->pool);
+  CallScratch S(c, s->stream);
   API_CUDA(defer_scratch(S), "closest scratch");
   RayArr R_trees{ray_trees, nullptr, ray_trees ? sizeof(int32_t) : 0};
   RayArr R_p{pts, nullptr, sizeof(double) * 3};
@@ -2701,7 +2722,7 @@ int xdgcu_segments_global(xdgcu_ctx* c, int32_t ipc_tree, int32_t element_tree, 
     return XDGCU_OK;
   }
   const bool mixed = precision == XDGCU_MIXED;
-  CallScratch S(st, c->pool);
+  CallScratch S(c, st);
   // the caller's arrays, or device images of host arrays
   const double* d_starts = starts;
   const double* d_ends = ends;
