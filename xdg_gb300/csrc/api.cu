@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cfloat>
 #include <cmath>
 #include <cstdio>
@@ -611,16 +612,18 @@ struct xdgcu_ctx {
   // global track loop on 1e6 tracks: 36.7 -> 33.0 ms); null: the default pool
   cudaMemPool_t pool = nullptr;
   int64_t keep_bytes = int64_t(8) << 30;
-  // most scratch bytes of a call (0: what the device has); stands in for a
-  // device without free memory in the tests of the paths for that
+  // most scratch bytes of the calls (0: what the device has), and what those
+  // with several blocks (CallScratch) hold; stands in for a device without free memory in the
+  // tests of the paths for that
   size_t scratch_limit = 0;
+  mutable std::atomic<size_t> scratch_held{0};
 };
 
 namespace {
 
 // Stream-ordered scratch of a call, from the context's pool.
 cudaError_t scratch_alloc(const xdgcu_ctx* c, void** p, size_t bytes, cudaStream_t s) {
-  if (c->scratch_limit && bytes > c->scratch_limit) return cudaErrorMemoryAllocation;
+  if (c->scratch_limit && c->scratch_held + bytes > c->scratch_limit) return cudaErrorMemoryAllocation;
   return c->pool ? cudaMallocFromPoolAsync(p, bytes, c->pool, s) : cudaMallocAsync(p, bytes, s);
 }
 
@@ -1136,15 +1139,22 @@ int begin_query(xdgcu_ctx* c, cudaStream_t st, unsigned long long** counters) {
 
 // Runs `body` with a.order set to the tracks sorted by decreasing length when
 // the batch is large enough (scratch allocated on the stream), else without.
+// Sets *no_memory (when given) if that scratch could not be had.
 template <typename Body>
-int with_length_order(xdgcu_ctx* c, WalkArgs& a, cudaStream_t s, Body body) {
+int with_length_order(xdgcu_ctx* c, WalkArgs& a, cudaStream_t s, Body body,
+                      bool* no_memory = nullptr) {
   if (c->walk_sort_min <= 0 || a.n < c->walk_sort_min || a.n >= ((int64_t)1 << 31)) return body();
   const size_t ord_bytes = ((sizeof(int32_t) * (size_t)a.n + 255) & ~(size_t)255);
   const size_t scr = walk_order_scratch_bytes(a.n);
   char* buf = nullptr;
-  API_CUDA(scratch_alloc(c, (void**)&buf, 256 + ord_bytes + scr, s), "walk order scratch");
+  cudaError_t e = scratch_alloc(c, (void**)&buf, 256 + ord_bytes + scr, s);
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // the failed allocation is not a pending launch error
+    if (no_memory) *no_memory = true;
+    return cuda_err(e, "walk order scratch");
+  }
   int32_t* const order = (int32_t*)(buf + 256);
-  cudaError_t e = walk_order(a.dist, a.n, order, buf + 256 + ord_bytes, scr, s);
+  e = walk_order(a.dist, a.n, order, buf + 256 + ord_bytes, scr, s);
   if (e != cudaSuccess) {
     cudaFreeAsync(buf, s);
     return cuda_err(e, "walk order");
@@ -1162,30 +1172,45 @@ int with_length_order(xdgcu_ctx* c, WalkArgs& a, cudaStream_t s, Body body) {
 struct CallScratch {
   const xdgcu_ctx* c;
   cudaStream_t st;
-  std::vector<void*> ptrs;
-  size_t held = 0;
+  std::vector<std::pair<void*, size_t>> blocks;
   CallScratch(const xdgcu_ctx* ctx, cudaStream_t s) : c(ctx), st(s) {}
-  ~CallScratch() {
-    for (void* p : ptrs) cudaFreeAsync(p, st);
+  ~CallScratch() { rewind(0); }
+  // what was taken after the first `count` blocks is freed
+  void rewind(size_t count) {
+    while (blocks.size() > count) {
+      cudaFreeAsync(blocks.back().first, st);
+      c->scratch_held -= blocks.back().second;
+      blocks.pop_back();
+    }
+  }
+  template <typename T>
+  void release(T** p) {
+    for (size_t k = 0; *p && k < blocks.size(); ++k) {
+      if (blocks[k].first != *p) continue;
+      cudaFreeAsync(blocks[k].first, st);
+      c->scratch_held -= blocks[k].second;
+      blocks.erase(blocks.begin() + (ptrdiff_t)k);
+      break;
+    }
+    *p = nullptr;
   }
   template <typename T>
   cudaError_t get(T** out, int64_t count) {
     *out = nullptr;
     void* p = nullptr;
     const size_t bytes = sizeof(T) * (size_t)std::max<int64_t>(1, count);
-    if (c->scratch_limit && held + bytes > c->scratch_limit) return cudaErrorMemoryAllocation;
     const cudaError_t e = scratch_alloc(c, &p, bytes, st);
     if (e != cudaSuccess) return e;
-    ptrs.push_back(p);
-    held += bytes;
+    blocks.emplace_back(p, bytes);
+    c->scratch_held += bytes;
     *out = static_cast<T*>(p);
     return cudaSuccess;
   }
 };
 
 // The K-strided walk buffer of the rounds (12 bytes per slot) holds at most
-// about this many bytes, or kSegStridedLeast where those cannot be had.  A
-// round that pauses no walk needs neither a second length order nor a second
+// about this many bytes, or kSegStridedLeast where the call's other scratch
+// needs the room (seg_strided_shrink).  A round that pauses no walk needs neither a second length order nor a second
 // end (1e6 tracks located and walked: 7.56 ms with 1 GiB, 7.16 with 4).
 constexpr int64_t kSegStridedBytes = int64_t(4) << 30;
 constexpr int64_t kSegStridedLeast = int64_t(1) << 30;
@@ -1240,9 +1265,24 @@ cudaError_t seg_strided_alloc(const xdgcu_ctx* c, int64_t n, CallScratch& S, Seg
     e = S.get(&B.sk_len, B.strided_cap);
     if (e == cudaSuccess) e = S.get(&B.sk_elem, B.strided_cap);
     if (e == cudaSuccess) return e;
-    cudaGetLastError();  // the failed allocation is not a pending launch error
+    S.release(&B.sk_len);  // the second attempt has the room of the first
+    cudaGetLastError();    // the failed allocation is not a pending launch error
   }
   return e;
+}
+
+// Gives back what the K-strided buffer of n tracks holds beyond its least
+// size, after another allocation of the call has failed; false where it holds
+// no more than that.  Its contents are lost.
+bool seg_strided_shrink(const xdgcu_ctx* c, int64_t n, CallScratch& S, SegWalkBufs& B) {
+  const int64_t least = seg_strided_cap(n, c->segments_walk_cap, kSegStridedLeast);
+  if (B.strided_cap <= least) return false;
+  S.release(&B.sk_len);
+  S.release(&B.sk_elem);
+  B.strided_cap = least;
+  const bool ok = S.get(&B.sk_len, least) == cudaSuccess && S.get(&B.sk_elem, least) == cudaSuccess;
+  cudaGetLastError();
+  return ok;
 }
 
 // One round of the capped single-pass walk for the m entries of the walk
@@ -1252,15 +1292,15 @@ cudaError_t seg_strided_alloc(const xdgcu_ctx* c, int64_t n, CallScratch& S, Seg
 // placement), the walk state advanced and the tracks still active appended to
 // act_next (seg_advance; walk_only: an ended walk finishes its track).
 // Synchronises `st` once, for the round's total.  On an allocation failure
-// sets *no_memory (when given).
-int seg_walk_round(xdgcu_ctx* c, bool mixed, const SegState& ss, const WalkArgs& geo,
-                   const SegWalkBufs& B, int32_t m, int32_t max_segs, bool walk_only,
-                   int32_t* act_next, int32_t* n_act, CallScratch& S, cudaStream_t st,
-                   bool* no_memory, SegRound* R) {
+// sets *no_memory; the walk state is then as it was.
+int seg_walk_try(xdgcu_ctx* c, bool mixed, const SegState& ss, const WalkArgs& geo,
+                 const SegWalkBufs& B, int32_t m, int32_t max_segs, bool walk_only,
+                 int32_t* act_next, int32_t* n_act, CallScratch& S, cudaStream_t st,
+                 bool* no_memory, SegRound* R) {
   auto get = [&](auto** p, int64_t count) -> bool {
     if (S.get(p, count) == cudaSuccess) return true;
     cudaGetLastError();  // the failed allocation is not a pending launch error
-    if (no_memory) *no_memory = true;
+    *no_memory = true;
     return false;
   };
   const int32_t K = seg_round_k(m, B.strided_cap, c->segments_walk_cap, max_segs);
@@ -1293,7 +1333,7 @@ int seg_walk_round(xdgcu_ctx* c, bool mixed, const SegState& ss, const WalkArgs&
   int rc = with_length_order(c, w, st, [&]() -> int {
     API_CUDA(launch_walk(mixed, c->face_order, w, st), "walk");
     return XDGCU_OK;
-  });
+  }, no_memory);
   if (rc) return rc;
   // the segments each track keeps (max_segs per walk), packed
   API_CUDA(seg_round_counts(ss, R->walk_t, m, B.wcnt, max_segs, R->off, st), "walk round counts");
@@ -1310,6 +1350,27 @@ int seg_walk_round(xdgcu_ctx* c, bool mixed, const SegState& ss, const WalkArgs&
                        w.sum_out, max_segs, R->off, R->dst_rel, act_next, n_act, st, walk_only),
            "walk advance");
   return XDGCU_OK;
+}
+
+// seg_walk_try, once more with the least strided buffer where the memory was
+// short of the rest.  Sets *no_memory (when given) if it still is.
+int seg_walk_round(xdgcu_ctx* c, bool mixed, const SegState& ss, const WalkArgs& geo,
+                   SegWalkBufs& B, int32_t m, int32_t max_segs, bool walk_only, int32_t* act_next,
+                   int32_t* n_act, CallScratch& S, cudaStream_t st, bool* no_memory, SegRound* R) {
+  const size_t held = S.blocks.size();
+  bool short_of = false;
+  int rc = seg_walk_try(c, mixed, ss, geo, B, m, max_segs, walk_only, act_next, n_act, S, st,
+                        &short_of, R);
+  if (short_of) {
+    S.rewind(held);
+    if (seg_strided_shrink(c, ss.n, S, B)) {
+      short_of = false;
+      rc = seg_walk_try(c, mixed, ss, geo, B, m, max_segs, walk_only, act_next, n_act, S, st,
+                        &short_of, R);
+    }
+  }
+  if (short_of && no_memory) *no_memory = true;
+  return rc;
 }
 
 // xdgcu_walk_elements_packed with one walk of every track instead of a count
@@ -1394,6 +1455,8 @@ int walk_packed_rounds(xdgcu_ctx* c, bool mixed, const WalkArgs& a, cudaStream_t
     std::swap(act, act_next);
   }
   // offsets from the tracks' totals, then every round's segments to their place
+  S.release(&B.sk_len);
+  S.release(&B.sk_elem);
   API_CUDA(seg_counts(ss, a.offsets, st), "packed walk totals");
   int64_t* sums = nullptr;
   get(&sums, scan_scratch_entries(n));
@@ -2805,6 +2868,12 @@ int xdgcu_segments_global(xdgcu_ctx* c, int32_t ipc_tree, int32_t element_tree, 
     int fo = 0, dev = 0;
     if (const char* msg = walk_args_for(c, &geo, &fo, &dev)) return set_err(XDGCU_ERR_STATE, msg);
   }
+  // runs `step`, again without the strided buffer's spare room if it failed
+  auto with_room = [&](auto step) -> int {
+    const int r = step();
+    if (r != XDGCU_ERR_CUDA || !seg_strided_shrink(c, n, S, B)) return r;
+    return step();
+  };
   int32_t round = 0;
   for (; m > 0 && round < max_rounds; ++round) {
     // paused walks resume; the other active tracks are located
@@ -2822,8 +2891,10 @@ int xdgcu_segments_global(xdgcu_ctx* c, int32_t ipc_tree, int32_t element_tree, 
       // the phased kernel locates faster (the global loop on three gapped
       // blocks: 3083 -> 3371 Msegs/s)
       API_CUDA(seg_gather_points(ss, loc, m_loc, pts, st), "segments gather");
-      rc = point_query(c, false, element_tree, nullptr, m_loc, pts, nullptr, eid, eidx, nullptr,
-                       precision, st, round > 0);
+      rc = with_room([&]() -> int {
+        return point_query(c, false, element_tree, nullptr, m_loc, pts, nullptr, eid, eidx, nullptr,
+                           precision, st, round > 0);
+      });
       if (rc) return rc;
       API_CUDA(seg_decide(ss, loc, m_loc, eid, eidx, B.walk_t, B.walk_start, n_walk, out_t, ray_org,
                           ray_dir, n_out, st),
@@ -2836,8 +2907,11 @@ int xdgcu_segments_global(xdgcu_ctx* c, int32_t ipc_tree, int32_t element_tree, 
       const int32_t m_out = h2[1];
       if (m_out > 0) {
         // ray_fire(ipc, r + u * TINY_BIT, u, INFTY, EXITING), then re-entry
-        rc = xdgcu_ray_fire(c, ipc_tree, nullptr, m_out, ray_org, ray_dir, nullptr, XDGCU_EXITING,
-                            nullptr, nullptr, t_hit, surf, face, nullptr, precision, st);
+        rc = with_room([&]() -> int {
+          return xdgcu_ray_fire(c, ipc_tree, nullptr, m_out, ray_org, ray_dir, nullptr,
+                                XDGCU_EXITING, nullptr, nullptr, t_hit, surf, face, nullptr,
+                                precision, st);
+        });
         if (rc) return rc;
         API_CUDA(seg_reenter(ss, out_t, m_out, t_hit, surf, face, c->d_bfe_face.p, c->d_bfe_elem.p,
                              c->n_bfe, (int32_t)c->n_tet, B.walk_t, B.walk_start, n_walk, st),
@@ -2861,6 +2935,8 @@ int xdgcu_segments_global(xdgcu_ctx* c, int32_t ipc_tree, int32_t element_tree, 
   }
   if (m > 0) API_CUDA(seg_stop_active(ss, act, m, XDGCU_RAY_WALK_LIMIT, st), "segments stop");
   // offsets from the per-track totals, then every round's segments to their place
+  S.release(&B.sk_len);
+  S.release(&B.sk_elem);
   API_CUDA(seg_counts(ss, d_off, st), "segments counts");
   {
     int64_t* sums = nullptr;
