@@ -492,10 +492,9 @@ int xdgcu_get_counters(xdgcu_ctx* ctx, int64_t counters[8]);
  *   "transport_event_wait" particle loop of xdgcu_transport_elements: lanes
  *                      whose events need the FP64 sample (collisions,
  *                      uncertain exits) that a warp gathers before it runs
- *                      them together, in batches that give every lane a
- *                      particle (1..32, default 4; smaller batches never wait,
- *                      mixed ones of eight particles a lane wait for at
- *                      least 8)
+ *                      them together (1..32, default 4: by the batch -- 4
+ *                      where every lane has a particle, 8 in mixed batches of
+ *                      eight particles a lane, and smaller ones do not wait)
  *   "trace_sort_min"   batches of at least this many rays (default 0 = never)
  *                      are traversed in a coherent order: sorted on the device
  *                      by tree, direction octant and the Morton code of the

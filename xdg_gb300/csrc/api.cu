@@ -33,6 +33,7 @@
 #include "cbound.h"
 #include "cobb.h"
 #include "imul64.cuh"
+#include "launch_rules.h"
 #include "queries.h"
 #include "segments.h"
 #include "walk.h"
@@ -563,7 +564,7 @@ struct xdgcu_ctx {
   int32_t surf_width8 = 0;            // some surface tree has 8-wide nodes
   int32_t surf_stack_bound = 0;       // largest (width - 1) * depth of the surface trees
   int32_t particle_event_wait = 20;  // particle_sim loop: lanes gathered before their events run
-  int32_t transport_event_wait = 4;  // walk_elements tool loop (mixed): the same
+  int32_t transport_event_wait = kTransportEventWait;  // walk_elements tool loop: the same
   int32_t leaf_max = 2;
   int32_t node_width = 4;        // children per BVH node (4 or 8) of trees built afterwards
   int32_t bvh_sah = 1;           // trees built afterwards: SAH collapse (1) or greedy (0)
@@ -3232,17 +3233,8 @@ int xdgcu_transport_elements(xdgcu_ctx* c, int64_t n, int32_t* elem_index, doubl
   t.n = n;
   t.mfp = mean_free_path;
   t.max_events = max_events;
-  // Waiting for fuller batches of collisions pays once every lane has a
-  // particle; before that the lanes that wait are what the launch waits for
-  // (ms with 1 / 2 / 4 lanes, mixed: 20,000 particles 11.5 / 12.1 / 12.2, 200,000
-  // 25.7 / 23.8 / 23.6; FP64: 14.8 / 15.6 / 15.8 and 34.0 / 32.2 / 32.6)
-  // and, mixed, fuller ones where a lane runs many particles (ms with 4 / 8 lanes:
-  // 600,000 particles 38.8 / 38.6, 1e6 53.6 / 51.7, 3e6 128.8 / 118.0; FP64
-  // 600,000 52.4 / 53.6).
   const bool mixed = precision == XDGCU_MIXED;
-  const int64_t full = (int64_t)device_sm_count() * 16 * 32;  // a particle for every lane
-  t.event_wait = n >= full ? c->transport_event_wait : 1;
-  if (mixed && n >= 8 * full) t.event_wait = std::max(t.event_wait, 8);
+  t.event_wait = transport_event_wait(c->transport_event_wait, mixed, n, device_sm_count());
   cudaStream_t st = (cudaStream_t)stream;
   if (kind == 1) {
     t.elem = elem_index;
