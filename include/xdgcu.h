@@ -463,7 +463,10 @@ int xdgcu_get_counters(xdgcu_ctx* ctx, int64_t counters[8]);
  *                      6, 7.03 with 8, 7.39 with 4 and 7.48 with 12
  *   "trace_flush_wait" number of lanes (1..32, default 4) whose rays wait
  *                      only on queued FP64 candidate tests before the warp
- *                      drains a partly filled queue
+ *                      drains a partly filled queue.  At the default the
+ *                      mixed particle loop of xdgcu_transport_surfaces waits
+ *                      for 12 lanes (32 - particle_event_wait, if that is
+ *                      less) in batches that give every lane a particle
  *   "trace_stack"      shared-memory traversal stack entries per ray (16..64,
  *                      steps of 8; default 40).  Deeper stacks take shared
  *                      memory and so resident blocks.  A launch raises it to

@@ -83,3 +83,7 @@ def test_surfaces(cuda, oracle, prec):
 
     for m in (1, full // BASE, full // BASE + 1):
         _check(run(m), want, m, m)
+    for flush, event in ((1, 24), (16, 1), (4, 32), (32, 32)):
+        x.rti.set_tuning("trace_flush_wait", flush)
+        x.rti.set_tuning("particle_event_wait", event)
+        _check(run(full // BASE + 1), want, full // BASE + 1, (flush, event))

@@ -556,7 +556,7 @@ struct xdgcu_ctx {
   int32_t trace_node_iters = 4;       // mixed precision
   int32_t trace_node_iters_fp64 = 2;  // all-FP64 path
   int32_t trace_node_iters_direct = 6;  // mixed launches reading their rays in place from host memory
-  int32_t trace_flush_wait = 4;
+  int32_t trace_flush_wait = kFlushWait;
   int32_t trace_stack = 40;      // shared-memory stack entries per lane
   int32_t trace_grab = 0;        // > 0: rays a warp takes from the device work queue; 0: see trace_queue
   int32_t trace_queue = 1;       // trace_grab 0: 1 by the batch (queue_grab_for), 0 one contiguous chunk per warp
@@ -3131,12 +3131,7 @@ int xdgcu_transport_surfaces(xdgcu_ctx* c, int64_t n, int32_t* tree, double* pos
   a.hist_cap = history_cap;
   a.event_wait = c->particle_event_wait;
   const bool mixed = precision == XDGCU_MIXED;
-  // Where every lane has a particle, the others' work covers a longer wait for
-  // fuller drains.  With event_wait 20 a wait for 12 lanes leaves two lanes
-  // searching at the least, and the pair is a sharp best (1e6 particles of
-  // the nested spheres, ms with 8 / 12 / 16 lanes: 73.9 / 70.4 / 72.2, 3e6 191 /
-  // 183 / 185, 200,000 29.2 / 28.2 / 28.2; event_wait 24 with 12: 85.7)
-  if (mixed && n >= (int64_t)device_sm_count() * 16 * 32) a.flush_wait = std::max(a.flush_wait, 12);
+  a.flush_wait = particle_flush_wait(a.flush_wait, a.event_wait, mixed, n, device_sm_count());
   cudaStream_t st = (cudaStream_t)stream;
   auto bind = [&](char* const* p) {
     a.p_tree = (int32_t*)p[0];

@@ -3,14 +3,27 @@
 // are.  Host code without CUDA, so that it can be checked as such.
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
 
 namespace xdgcu {
 
+constexpr int32_t kFlushWait = 4;           // trace_flush_wait
 constexpr int32_t kTransportEventWait = 4;  // transport_event_wait
 
 // a particle for every lane of 16 warps on each of `sms` SMs
 inline int64_t full_batch(int sms) { return (int64_t)sms * 16 * 32; }
+
+// SurfArgs::flush_wait of the surface particle loop.  Where every lane has a
+// particle, the others' work covers a longer wait for fuller drains.  With
+// event_wait 20 a wait for 12 lanes leaves two lanes searching at the least,
+// and beyond that sum of 32 lanes nothing is left (1e6 particles of the
+// nested spheres, ms with 8 / 12 / 16 lanes: 73.9 / 70.4 / 72.2, 3e6 191 / 183 /
+// 185, 200,000 29.2 / 28.2 / 28.2; event_wait 24 with 12: 85.7).
+inline int32_t particle_flush_wait(int32_t key, int32_t event_wait, bool mixed, int64_t n, int sms) {
+  if (key != kFlushWait || !mixed || n < full_batch(sms)) return key;
+  return std::max(key, std::min(12, 32 - event_wait));
+}
 
 // TransportArgs::event_wait.  Waiting for fuller batches of collisions pays
 // once every lane has a particle; before that the lanes that wait are what
