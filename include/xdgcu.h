@@ -678,8 +678,10 @@ int xdgcu_autotune_trace(xdgcu_ctx* ctx, int32_t query, int32_t tree, const int3
  * walk_queue (mixed precision only), walk_flush_wait and, for samples of at
  * least 16,384 tracks, walk_sort_min, on a sample of xdgcu_walk_elements
  * (device arrays, strided output of max_segs per track allocated by the
- * tuner).  Same search, timing and result check as xdgcu_autotune_trace;
- * when the length order wins, walk_sort_min is set to max(16384, n/4). */
+ * tuner).  Same search, timing and result check as xdgcu_autotune_trace.
+ * When the length order wins, walk_sort_min keeps its value (its default
+ * where it was 0; n where it was above n), so that smaller batches keep the
+ * order too. */
 int xdgcu_autotune_walk(xdgcu_ctx* ctx, int64_t n, const int32_t* start_index,
                         const double* start, const double* u, const double* distance,
                         int32_t max_segs, int32_t precision, int32_t reps, double* best_ms);
