@@ -411,7 +411,7 @@ int xdgcu_transport_surfaces(xdgcu_ctx* ctx, int64_t n, int32_t* tree, double* p
  *     allocating walk uses for batches of at least `walk_sort_min` tracks
  *     (that order sorts the tracks into scratch memory), so
  *     `walk_sort_min` has no effect here: the results are the same, and
- *     it runs at about half the allocating walk's rate (2323 against 4664
+ *     it runs at about half the allocating walk's rate (3660 against 7510
  *     Msegs/s on 1e6 tracks of a 750,000-tet cube);
  *   - the first call on a device looks up the static array's device address
  *     (cudaGetSymbolAddress); make that first call before any stream capture.
@@ -448,19 +448,21 @@ int xdgcu_get_counters(xdgcu_ctx* ctx, int64_t counters[8]);
  *                      of the warp-synchronous traversal, mixed precision
  *                      (1..64, default 4; the FP64 path's default is 2).  On
  *                      the nested spheres every query ran fastest with 4 (1e7
- *                      rays, ms with 2/4/8/16 steps: ray_fire 7.36/6.50/
- *                      6.70/8.03, point_in_volume 7.05/6.23/6.41/7.71,
- *                      occluded 5.52/4.90/5.15/6.26, find_volume 22.6/22.1/
- *                      24.5/29.9)
+ *                      rays, ms with 2/4/8/16 steps: ray_fire 6.06/5.37/
+ *                      5.63/6.77, point_in_volume 5.88/5.23/5.49/6.63,
+ *                      occluded 5.02/4.44/4.60/5.51, find_volume 17.2/16.3/
+ *                      18.3/22.6)
  *   "trace_node_iters_fp64"  the same for the all-FP64 path (1e6 rays of the
- *                      nested spheres, ms with 1/2/3/4/6 steps: 1.82/1.74/
- *                      1.74/1.80/1.94)
+ *                      nested spheres, ms with 1/2/3/4/6 steps: 1.75/1.68/
+ *                      1.69/1.75/1.89)
  *   "trace_node_iters_direct"  the same for mixed calls whose rays the
  *                      kernel reads in place from host memory (host_direct;
- *                      default 6).  The best setting differs: 1e7 rays of
- *                      the nested spheres ran 6.45 ms from device arrays
- *                      with 4 steps (6.64 with 8) but in place 6.93 ms with
- *                      6, 7.03 with 8, 7.39 with 4 and 7.48 with 12
+ *                      default 6).  Over the host link more steps pay, the
+ *                      more the larger the batch: nested spheres in place, ms
+ *                      with 4/6/8/12 steps: 1e5 rays 0.22/0.20/0.20/0.21, 1e7
+ *                      8.94/8.36/8.08/7.81 (5.37/5.38/5.63 with 4/6/8 from
+ *                      device arrays; the link's rate varies by half
+ *                      from run to run)
  *   "trace_flush_wait" number of lanes (1..32, default 4) whose rays wait
  *                      only on queued FP64 candidate tests before the warp
  *                      drains a partly filled queue.  At the default the
@@ -522,9 +524,10 @@ int xdgcu_get_counters(xdgcu_ctx* ctx, int64_t counters[8]);
  *                      face tests before the warp runs a partly filled round
  *   "walk_sort_min"    batches of at least this many tracks (default 16384;
  *                      0 = never) are walked longest first: the tracks are
- *                      sorted by length on the device and dealt round-robin
- *                      to warps, so warps end on short tracks.  Results do not
- *                      depend on it.
+ *                      sorted by length on the device and the warps take
+ *                      them 32 at a time from a counter, so that the lanes
+ *                      of a warp, and the warps, end together.  Results do
+ *                      not depend on it.
  *   "trace_edge_table" ray_fire / point_in_volume / occluded /
  *                      find_volume / particle loop: 1 (default) takes each
  *                      triangle's ray-independent FP64 terms (edge vectors,
@@ -542,33 +545,34 @@ int xdgcu_get_counters(xdgcu_ctx* ctx, int64_t counters[8]);
  *                      before the warp's lanes bound and test the triangles of
  *                      the leaves they hold together (1..64, default 4;
  *                      with the points in Morton order 4 ran 1e6 points in
- *                      15.4 ms, 8 in 16.6, 2 in 15.6, 16 in 17.4)
- *   "closest_node_steps_fp64"  the same for the all-FP64 closest (default 1)
+ *                      5.31 ms, 8 in 5.64, 2 in 5.39, 16 in 6.11)
+ *   "closest_node_steps_fp64"  the same for the all-FP64 closest (default 1;
+ *                      1e6 points 52.4 ms, 50.1 with 2, 54.7 with 4)
  *   "closest_step_budget"  closest: node records and triangles a lane visits
  *                      for one point (default 1024; 0 = no limit) before the
  *                      point is left to a second kernel that searches it with
  *                      a whole warp.  A point almost equidistant from many
  *                      triangles (the centre of a sphere) otherwise holds one
- *                      lane, and the launch, for thousands of steps (1e6
- *                      points of the nested spheres: 25.8 -> 32.0 Mpoints/s
- *                      mixed, 4.45 -> 6.23 FP64).  Results do not depend on
- *                      it
+ *                      lane, and the launch, for as many steps.  With the
+ *                      oriented boxes that is rare: 1e6 points of the nested
+ *                      spheres take 5.30 ms, 5.27 without a limit (FP64 52.4
+ *                      and 54.0).  Results do not depend on it
  *   "closest_sort_min"  closest: batches (or staged chunks) of at least this
  *                      many points run in the order of [tree | Morton code
  *                      of the point] (default 65536; 0 = the caller's
  *                      order), so that the points of a warp share their
  *                      upper nodes and take similar work; the order is
  *                      computed in the call's scratch (one radix sort).
- *                      1e6 points of the nested spheres: 35.9 -> 60.5
- *                      Mpoints/s mixed, 155 -> 92 ms FP64.  Results do not
- *                      depend on it
- *   "find_sort_min"    the same for find_element (default 65536; 1e6 points
- *                      of the 750,000-tet cube: 0.723 -> 0.700 ms mixed,
- *                      8.74 -> 8.07 ms FP64).  The ray queries' own order
- *                      (trace_sort_min) stays off by default: with it,
- *                      point_in_volume of 1e7 points took 15.9 instead of
- *                      6.7 ms, the warps' contiguous shares of similar rays
- *                      being unequal work
+ *                      1e6 points of the nested spheres: 7.94 -> 5.32 ms
+ *                      mixed, 94.7 -> 52.4 ms FP64.  Results do not depend
+ *                      on it
+ *   "find_sort_min"    the same for find_element (default 65536; 1e6 / 2e6
+ *                      points of the 750,000-tet cube, in the caller's order
+ *                      -> sorted: 0.56 -> 0.61 / 1.04 -> 1.05 ms mixed, 1.56 ->
+ *                      1.35 / 2.92 -> 2.42 ms FP64).  The ray queries' own
+ *                      order (trace_sort_min) stays off by default: with it,
+ *                      point_in_volume of 1e7 points took 5.76 instead of
+ *                      5.24 ms
  *   "find_node_steps_fp64"  the same for the all-FP64 find_element (default
  *                      4: 50,021 points 230 us, 16 258; 2e6 2.39 ms, 2 2.59),
  *                      and for the mixed one when it runs in phases
@@ -596,12 +600,12 @@ int xdgcu_get_counters(xdgcu_ctx* ctx, int64_t counters[8]);
  *                      count walk, then an emit walk), without the temporary
  *                      memory of the rounds.  Results do not depend on it
  *   "find_element_phased"  mixed find_element: 0 (default) runs one lane per
- *                      point on its own, the faster for points inside tets
- *                      (1409 against 1249 Mpoints/s on 1e6 uniform points of
- *                      a 750,000-tet cube); 1 runs the warp's lanes in step
+ *                      point on its own, as fast or faster for points inside
+ *                      tets (1e6 uniform points of a 750,000-tet cube 0.606
+ *                      and 0.618 ms); 1 runs the warp's lanes in step
  *                      with their exact FP64 tests together, the faster for
  *                      points on tet faces, where the FP32 filter decides
- *                      little (445 against 198 Mpoints/s on the cube's faces).
+ *                      little (1e6 on the cube's faces 0.734 and 0.448 ms).
  *                      xdgcu_segments_global locates in phases after its
  *                      first round whatever this says.  Results do not
  *                      depend on it

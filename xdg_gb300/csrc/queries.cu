@@ -821,10 +821,10 @@ __device__ __forceinline__ bool in_box64(const Node64* np, int k, d3 p) {
 }
 
 // One thread per point, each on its own: the mixed path, whose FP32 filter
-// decides nearly every tet of an interior point, runs faster this way (1409
-// against 1249 Mpoints/s in warp-synchronous phases, 1e6 uniform points in
-// the 750,000-tet cube).  For points on the cube's faces, where most tets
-// take the exact test, the phases win: 445 against 198 Mpoints/s.
+// decides nearly every tet of an interior point, runs no slower this way (1e6
+// uniform points in the 750,000-tet cube 0.606 ms, 0.618 in warp-synchronous
+// phases; 50,000 92 and 94 us).  For points on the cube's faces, where most
+// tets take the exact test, the phases win: 1e6 0.734 and 0.448 ms.
 template <bool MIXED>
 __global__ void __launch_bounds__(kBlock) k_find_element_lane(PointArgs a) {
   const int64_t i = point_index(a);

@@ -903,8 +903,11 @@ cudaError_t launch_minb(const SurfArgs& a, cudaStream_t st, int slot) {
         occupancy_cached(g_blocks_per_sm[slot][kVar][a.stack / 8], kern, kTBlock, smem, per_sm);
     if (e != cudaSuccess) return e;
   }
-  // (a ray of these modes waits for memory; the others wait for the FP64 unit
-  // and do better with fuller warps)
+  // (a ray of the spread modes waits for memory; the others wait for the FP64
+  // unit and do better with fuller warps.  The particle loop's warps always
+  // take 32 from the work queue: there the rule only adds blocks, whose first
+  // warps then hold the particles on more SMs and whose others end at once --
+  // 2,000 particles 10.7 ms, 10,000 13.4; 10.8 and 13.6 without)
   constexpr bool restarts = MODE == MODE_FIND_VOLUME || MODE == MODE_ALL_VOLUMES;
   constexpr bool spread = restarts || (MIXED && MODE != MODE_PARTICLE);
   const int lanes = lanes_per_warp(a.n, spread ? kSpreadWarps : kFp64Warps);
