@@ -261,9 +261,9 @@ int xdgcu_walk_elements(xdgcu_ctx* ctx, int64_t n, const int32_t* start_index,
  * walked once, in rounds of walks capped at 16..512 segments per track: a
  * walk that reaches the cap pauses and the next round resumes it where it
  * stopped; each round's segments wait in temporary device memory (about the
- * output's size, plus a buffer of up to 4 GiB, allocated on `stream` from
- * the context's scratch pool, "scratch_keep_bytes") until the offsets are
- * known.  Where that memory cannot be
+ * output's size, plus a buffer of up to 4 GiB, cut to 1 GiB where the rest
+ * does not fit beside it, allocated on `stream` from the context's scratch
+ * pool, "scratch_keep_bytes") until the offsets are known.  Where that memory cannot be
  * had, or with the tuning key "packed_walk_passes" = 2, the tracks are walked
  * twice instead (count, then emit at the scanned offsets), which needs only
  * the scan's scratch.  The results are the same either way. */
@@ -293,7 +293,7 @@ int xdgcu_set_boundary_face_elements(xdgcu_ctx* ctx, int64_t n, const int32_t* f
  * one ray_fire launch for those outside the mesh and one walk launch, with
  * the bookkeeping in device kernels.  A round's walk emits at most K
  * segments per track (K = 16..512, chosen so the round buffer stays near
- * 4 GiB); a longer walk pauses and the next round resumes it from where it
+ * 4 GiB, or 1 GiB where the call's other temporary memory needs the room); a longer walk pauses and the next round resumes it from where it
  * stopped, with the same operations as one uninterrupted walk.
  * Output as xdgcu_walk_elements_packed: track i's segments (element MESH
  * ids, lengths) at offsets[i] .. offsets[i+1]-1 of arrays of `capacity`
