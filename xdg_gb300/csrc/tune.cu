@@ -244,7 +244,7 @@ int xdgcu_autotune_trace(xdgcu_ctx* c, int32_t query, int32_t tree, const int32_
       {"trace_stack", {32, 40, 48, 64}},
       {mixed ? "trace_node_iters" : "trace_node_iters_fp64", {1, 2, 4, 8, 16}},
       {"trace_flush_wait", {4, 8, 16, 32}},
-      {"trace_grab", {0, 64, 256, 1024, 4096}},
+      {"trace_grab", {0, 64, 256, 1024, 4096}},  // 0: by the batch (trace_queue)
   };
   if (n >= 65536) knobs.push_back({"trace_sort_min", {0, n}});
   // tree shapes: the current one first, then (tune_tree) every node width
